@@ -205,22 +205,22 @@ int umwm_gpu_get_screen(double* out, long n, long* rows);
  * then runs host-driven), "device" (CUDA device of the next initialize),
  * "stress_ocn" (run stress('ocn') after every outer step: the last substep
  * of each step keeps its source terms, three more spectrum-sized arrays),
- * "direction_groups" (2: each point's directions in two half-turn groups
- * per warp lane pair; 4: four quarter-turn groups, twice the CTAs; needs
- * pm % 4 == 0 and pm/4 in {4, 6, 8, 9, 12}; initialize picks 4 below 3
- * 64-point tiles per SM and 2 above; results differ by summation order
- * only), "advect_groups" (the same for the propagation kernel alone), "gust_seed" (seed of the wind gust draws when
+ * "direction_groups" (2: a block of 32 points' levels go to the few warps
+ * that suit large models; 4: to more of them; 4 needs pm % 4 == 0 and pm/4
+ * in {4, 6, 8, 9, 12}; initialize picks 4 up to one 64-point tile per SM and
+ * 2 above; results do not change), "advect_groups" (the same for the
+ * propagation kernel alone), "gust_seed" (seed of the wind gust draws when
  * the namelist's gustiness > 0, umwm_forcing.F90:49-61; default 1: the
  * draws are a function of seed, substep, grid cell and component, so a run
  * repeats with its seed), "phys_groups" / "integ_groups" (the mapping of the
  * dts pre-pass or the integration alone), "minb_phys" / "minb_integ" /
- * "minb_advect" (resident CTAs per SM the kernel's register budget is sized
- * for; 0 or a budget without a compiled instance: the default) and
- * "pf_phys" / "pf_integ" / "pf_advect" (frequency levels each kernel
- * prefetches into L2 ahead), "advect_tma" / "phys_tma" (the propagation /
- * dts pre-pass of the two-group 36-direction mapping stage each level's own
- * rows in shared memory with bulk copies: advect_tma 1 the E* and e rows,
- * 2 the E* rows only; phys_tma 1 the e rows; results do not change),
+ * "minb_advect" (the kernel instance: resident CTAs per SM its register
+ * budget is sized for; 0 or a budget without a compiled instance: the
+ * default) and "pf_phys" / "pf_integ" / "pf_advect" (frequency levels each
+ * kernel prefetches into L2 ahead), "phys_tma" (default 1: the dts pre-pass
+ * stages its rows in shared memory with bulk copies; 36 directions; results
+ * do not change), "advect_tma" (accepted; the propagation stages its rows in
+ * every form),
  * "autotune" (0 off; 1: from the next substep
  * on, time the register budgets and prefetch distances of the three
  * spectral kernels on the model's own substeps, round-robin, and keep the

@@ -7,12 +7,18 @@
 // tile belongs to one member.  The index space is grouped in NB blocks of 32
 // consecutive points (ldN = 32 NB):
 //   spectrum arrays E, ES (= E* after the source half-step), EF:
-//       [o][j/32][p][32]: one frequency of one 32-point block is a
-//       contiguous P*128-byte region; within it direction p is a 128-byte
-//       line of 32 consecutive points, so a warp reading one bin for 16 or
-//       32 points is one coalesced access and every direction offset is a
-//       compile-time immediate
-//   per-(o,i) tables TAB: [o][j/32][table][32], tables T_* below
+//       [j/32][o][p/4][32][4]: a 32-point block's whole spectrum is one
+//       contiguous region of O*P*128 bytes, one frequency of it P*128 bytes;
+//       within that four directions of a point are 16 consecutive bytes, so a
+//       warp (lane = point) reads four directions of 32 points as one 512-byte
+//       access, a thread gets its direction pairs in register pairs, and every
+//       direction offset is a compile-time immediate.  The blocks in flight
+//       and their neighbours lie in a window of memory that few large pages
+//       cover, whichever levels their warps are at
+//   per-(o,i) tables TAB: [j/32][o][table][32], tables T_* below
+//   mss prefix MSS: [j/32][o][3][32], the sums A, B, C over the levels below o
+//       of k^3 dk dth/2 sum_p e (1, cos 2th, sin 2th); kept with E by whoever
+//       writes E (the propagation, and k_mss after a state is set)
 //   per-point arrays: [ldN]; all-point (land included) arrays: [imm]
 #pragma once
 #include <cstdint>
@@ -23,26 +29,26 @@ constexpr int MAX_OM = 64;
 constexpr int MAX_PM = 72;
 constexpr int MAX_LM = 100;
 
-// per-(o,i) table rows (stored per frequency o, then table, then point);
-// the rows the propagation reads come first (T_ADV_ROWS of them), so that
-// it prefetches only those
+// per-(o,i) table rows (stored per frequency o, then table, then point)
 enum TableRow {
-  T_K = 0,      // wavenumber k                       umwm_init.F90:1473
+  T_CG0 = 0,    // group velocity cg0 (ghost = min)   umwm_init.F90:1494, :1653-1656
+  T_KDK,        // k dk                               :1505
+  T_K3DK,       // k^3 dk                             :1506
   T_CP0,        // phase speed cp0 (ghost = min)      :1493, :1653-1656
-  T_CG0,        // group velocity cg0 (ghost = min)   :1494, :1653-1656
   T_LOGL2Z,     // log(l2/z), capped                  :1530-1533
   T_FKOVG,      // f k / g                            :1507
-  T_KDK,        // k dk                               :1505
-  T_K4,         // k^4                                :1503
-  T_K3DK,       // k^3 dk                             :1506
-  T_COTHKD,     // coth(0.2 kd)                       :1508
+  T_K,          // wavenumber k                       :1473
   T_SBF,        // bottom friction+percolation        :1510-1511
   T_SDV,        // viscous dissipation                :1512
+  T_COTHKD,     // coth(0.2 kd)                       :1508
   T_BF1R,       // Snl weight to o+1                  :1523
   T_BF2R,       // Snl weight to o+2                  :1524
   T_COUNT
 };
-constexpr int T_ADV_ROWS = T_KDK + 1;  // rows 0 .. T_KDK: all the propagation and stress read
+// rows 0 .. T_FKOVG: all the propagation and stress read; rows T_CP0 .. T_BF2R:
+// what the source terms read (k^4 is formed from k)
+constexpr int T_ADV_ROWS = T_FKOVG + 1;
+constexpr int T_SRC0 = T_CP0, T_SRC_ROWS = T_BF2R + 1 - T_CP0;
 
 constexpr int TILE = 64;  // wet points of a tile (a member's points start on a tile boundary)
 
@@ -60,8 +66,9 @@ constexpr int TILE = 64;  // wet points of a tile (a member's points start on a 
 #define UMWM_PF_DIST_ADV 1
 #endif
 
-// Direction groups per point of the spectral kernels: 4 quarter-turn groups
-// when pm % 4 == 0 and pm/4 is a supported group size, else 2 half-turn groups.
+// Direction counts with the small-model split of the levels over more warps
+// (options "direction_groups" and the like, value 4) and with direction
+// constants from a quarter turn.
 __host__ __device__ constexpr bool quarter_groups(int pm) {
   return pm % 4 == 0 && (pm / 4 == 4 || pm / 4 == 6 || pm / 4 == 8 || pm / 4 == 9 || pm / 4 == 12);
 }
@@ -72,6 +79,7 @@ struct Member;
 struct Params {
   int Ntot, ldN, NB, O, P, NMtot, lm;
   int nmem;              // members
+  int nsm;               // SMs of the device
   int ntiles;            // CTA tiles of TILE points over the whole index space
   const Member* mem;     // [nmem]
   const int* tile_mem;   // member of each tile [ntiles]
@@ -85,7 +93,7 @@ struct Params {
   unsigned gust_seed;   // seed of the gust draws (option "gust_seed")
   int winds, currents, air_density, water_density, seaice, restart, curvilinear, isglobal;
   int ice_possible;  // fice can exceed fice_lth somewhere
-  int groups4;       // the integration uses 4 quarter-turn direction groups (option "direction_groups")
+  int groups4;       // the integration splits a block's levels over more warps (option "direction_groups" 4)
   int groups4_phys;  // the dts pre-pass does (options "direction_groups", "phys_groups")
   int adv_groups4;   // the propagation kernel does (options "direction_groups", "advect_groups")
   // Launch configuration of the three spectral kernels, chosen by the
@@ -96,16 +104,17 @@ struct Params {
   int minb_phys, minb_integ, minb_adv;
   int pf_phys, pf_integ, pf_adv;
   int count_cut;     // the propagation counts the bins its non-negativity cut changes (Global::cut_count)
-  int swsign;        // the first pm/2 directions have sin th < 0, and cos th < 0 exactly for the first pm/4
-                     // (pm % 4 == 0): the two-group flux takes one upwind term per slot pair
-  int adv_tma;       // the propagation stages its own rows with bulk copies (k_advect_tma; option "advect_tma")
-  int phys_tma;      // the dts pre-pass does (k_source_tma; option "phys_tma")
+  int swsign;        // the first pm/2 directions have sin th < 0, and of them the first pm/4 (and the last
+                     // pm/4 of all) cos th < 0: the propagation takes its upwind sides from the index
+  int adv_tma;       // option "advect_tma" (no effect: the propagation stages its rows in every form)
+  int phys_tma;      // the dts pre-pass stages its rows with bulk copies (option "phys_tma")
   float f[MAX_OM], dom[MAX_OM];
   float th[MAX_PM], cth[MAX_PM], sth[MAX_PM], c2th[MAX_PM], s2th[MAX_PM];
-  float shs[MAX_PM], chs[MAX_PM];  // (sin th(p) + sin th(p+1)) / 2, the same for cos: the edge between p and p+1
-  // max(cos th, 0), min(cos th, 0), max(sin th, 0), min(sin th, 0): the
-  // upwind weights of propagation (umwm_advection.F90:34-47)
-  float cthp[MAX_PM], cthm[MAX_PM], sthp[MAX_PM], sthm[MAX_PM];
+  // The spectral kernels' direction constants: those of the directions of a
+  // quarter (or half) turn, turned exactly to the others, so that opposite
+  // directions (and, with quarters, perpendicular ones) have the same rounding;
+  // and the mean sin and cos over the edge between p and p+1
+  float dcth[MAX_PM], dsth[MAX_PM], dc2th[MAX_PM], ds2th[MAX_PM], shs[MAX_PM], chs[MAX_PM];
   float depth[MAX_LM];
 };
 
@@ -160,7 +169,8 @@ struct Global {
 
 struct Ptrs {
   float *E, *ES, *EF;  // spectrum arrays (EF aliases E: each bin is read and then overwritten by one thread)
-  const float* TAB;     // [O][T_COUNT][ldN]
+  const float* TAB;     // [NB][O][T_COUNT][32]
+  float* MSS;           // [NB][O][3][32]
   // wet-point arrays [ldN]
   const int *ie, *iw, *in, *is;      // aliased neighbours (global index; the member's ghost for land)
   const int *iie, *iiw, *iin, *iis;  // true neighbours (global all-point index)
@@ -224,10 +234,12 @@ __host__ __device__ inline float gust_uniform(unsigned seed, unsigned substep, u
 
 // element offsets in the blocked layouts
 __host__ __device__ inline size_t sidx(const Params& prm, int o, int p, int j) {
-  return ((size_t)(o * prm.NB + (j >> 5)) * prm.P + p) * 32 + (j & 31);
+  return ((size_t)(j >> 5) * prm.O + o) * prm.P * 32 + (p >> 2) * 128 + (j & 31) * 4 + (p & 3);
 }
 __host__ __device__ inline size_t tidx(const Params& prm, int o, int t, int j) {
-  return ((size_t)(o * prm.NB + (j >> 5)) * T_COUNT + t) * 32 + (j & 31);
+  return (((size_t)(j >> 5) * prm.O + o) * T_COUNT + t) * 32 + (j & 31);
 }
+// offset of direction p from direction 0 of the same bin row
+__host__ __device__ constexpr int poff(int p) { return (p >> 2) * 128 + (p & 3); }
 
 }  // namespace umwm

@@ -63,6 +63,15 @@ __device__ __forceinline__ float max_nan0(float x) {
   return r;
 }
 
+__device__ __forceinline__ float2 f2(float a) { return make_float2(a, a); }
+
+// max(x, lo) with NaN kept
+__device__ __forceinline__ float max_nan(float x, float lo) {
+  float r;
+  asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(x), "f"(lo));
+  return r;
+}
+
 // Sin of one bin from x = U cos(wdir - th) - cp0 - uc cos th - vc sin th,
 // umwm_source_functions.F90:39-80, with its factors folded: the reference
 // forms sin_fac |x| x, then multiplies by shelt/sin_fac where positive, by
@@ -80,28 +89,6 @@ __device__ __forceinline__ float sin_fold(const Params& prm, float shelt, float 
   return s;
 }
 
-// sin_fold of the two directions k, k+1 of one lane, with x formed as the
-// scalar callers form it (U cw - cp0 - ucg cos th - vcg sin th) and the
-// affine parts in packed f32x2 arithmetic (the integration's pairs: 2.29 ->
-// 2.28 ms at 1000x1000; in the pre-pass and the propagation it measured no
-// faster)
-__device__ __forceinline__ float2 sin_fold2(const Params& prm, float shelt, float U, float2 cw, float ucg, float vcg,
-                                            float2 cth, float2 sth, float cp0, float gl, bool tail) {
-  float2 x = __ffma2_rn(make_float2(U, U), cw, make_float2(-cp0, -cp0));
-  x = __ffma2_rn(make_float2(-ucg, -ucg), cth, x);
-  x = __ffma2_rn(make_float2(-vcg, -vcg), sth, x);
-  const float2 a = make_float2(x.x * fabsf(x.x), x.y * fabsf(x.y));
-  const float2 f = make_float2(x.x > 0.f ? shelt : (cw.x > 0.f ? prm.sin_neg2 : prm.sin_neg1),
-                               x.y > 0.f ? shelt : (cw.y > 0.f ? prm.sin_neg2 : prm.sin_neg1));
-  float2 s = __fmul2_rn(__fmul2_rn(a, f), make_float2(gl, gl));
-  if (tail) s = make_float2(fmaxf(s.x, 0.f), fmaxf(s.y, 0.f));
-  return s;
-}
-
-#ifndef UMWM_PREFETCH_TAB
-#define UMWM_PREFETCH_TAB 1  // the spectral kernels also prefetch the block's table rows with the spectrum
-#endif
-
 // 2^x through the SFU (ex2.approx.ftz)
 __device__ __forceinline__ float ex2_approx(float x) {
   float y;
@@ -109,15 +96,72 @@ __device__ __forceinline__ float ex2_approx(float x) {
   return y;
 }
 
-// 4-byte asynchronous copy global -> shared (cp.async), its group commit and
-// wait (the wait ends when this thread's copies have landed)
-__device__ __forceinline__ void cp_async4(float* smem, const float* gmem) {
-  const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(sa), "l"(gmem) : "memory");
+// bulk prefetch of a contiguous, 16-byte aligned range into L2 (sizes are multiples of 16 bytes)
+__device__ __forceinline__ void bulk_prefetch_l2(const void* p, unsigned bytes) {
+  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
 }
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+// k^4 rounded once (the products' errors carried), as the host's tables have powers
+__device__ __forceinline__ float pow4(float k) {
+  const float h = __fmul_rn(k, k), l = fmaf(k, k, -h), q = __fmul_rn(h, h);
+  return __fadd_rn(q, fmaf(2.f * h, l, fmaf(h, h, -q)));
+}
+
+// The direction constants of four directions: cos and sin of th and of 2 th,
+// and the mean sin and cos over the edge to the next direction.  A CTA copies
+// them to shared memory ([pm/4] of them, float4 each): the packed arithmetic
+// takes register pairs, and holding pm of them over the levels (where the
+// compiler puts loop-invariant constants) would cost the registers.
+enum DirRow { DIR_C = 0, DIR_S, DIR_C2, DIR_S2, DIR_SH, DIR_CH, DIR_ROWS };
+template <int NP>
+__device__ __forceinline__ void dir_fill(const Params& prm, float* d) {  // then a CTA barrier
+  for (int p = threadIdx.x; p < NP; p += blockDim.x) {
+    float* r = d + (p >> 2) * (4 * DIR_ROWS) + (p & 3);
+    r[4 * DIR_C] = prm.dcth[p];
+    r[4 * DIR_S] = prm.dsth[p];
+    r[4 * DIR_C2] = prm.dc2th[p];
+    r[4 * DIR_S2] = prm.ds2th[p];
+    r[4 * DIR_SH] = prm.shs[p];
+    r[4 * DIR_CH] = prm.chs[p];
+  }
+}
+// (volatile: read where it is used)
+struct F2x2 {
+  float2 a[2];
+};
+__device__ __forceinline__ F2x2 dir4(uint32_t dirs, int q, int row) {
+  F2x2 v;
+  asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+               : "=f"(v.a[0].x), "=f"(v.a[0].y), "=f"(v.a[1].x), "=f"(v.a[1].y)
+               : "r"(dirs + (uint32_t)(q * DIR_ROWS + row) * 16u));
+  return v;
+}
+
+// cos(wdir - th) of directions 4q0 .. 4q1 - 1 of this lane's point into shared
+// memory, four directions per float4: cw[q * 32 + lane].  (Formed from the
+// rounded angle as the reference does: x = U cos(wdir - th) - cp0 - ...
+// cancels, and products of cos wdir and cos th round differently there.)
+__device__ __forceinline__ void cw_fill(const Params& prm, float wdir, int q0, int q1, int step, float4* cw) {
+  const int lane = threadIdx.x & 31;
+  for (int q = q0; q < q1; q += step)
+    cw[q * 32 + lane] = make_float4(cosf(wdir - prm.th[4 * q]), cosf(wdir - prm.th[4 * q + 1]),
+                                    cosf(wdir - prm.th[4 * q + 2]), cosf(wdir - prm.th[4 * q + 3]));
+}
+
+// The mss prefix of sum m (0: A, 1: B, 2: C) of block blk, one lane per point:
+// MSS[o] = the levels' sums below o, from v[o * stride + m * 32 + lane] in
+// shared memory, added in the order of the levels.
+__device__ __forceinline__ void mss_prefix(const Params& prm, const Ptrs& P, int blk, int m, const float* v,
+                                           int stride) {
+  const int lane = threadIdx.x & 31;
+  float a = 0.f;
+  float* out = P.MSS + (size_t)blk * prm.O * 96 + m * 32 + lane;
+#pragma unroll 4
+  for (int o = 0; o < prm.O; ++o) {
+    out[(size_t)o * 96] = a;
+    a += v[(size_t)o * stride + m * 32 + lane];
+  }
+}
 
 // stress_tail, umwm_stress.F90:300-311
 __device__ __forceinline__ float stress_tail(float w, float kmax) {
@@ -161,15 +205,5 @@ __device__ __forceinline__ bool adv_mbar_wait(uint32_t bar, uint32_t parity, lon
     if (clock64() - t0 > limit_cycles) return false;
   return true;
 }
-
-// Own-row staging of the TMA forms of the propagation and the dts pre-pass:
-// each level's rows of the CTA's 64 points (two blocks, one contiguous
-// region per array) land in shared memory by bulk copies issued one level
-// ahead, into two alternating buffers, each completing on its own mbarrier.
-struct OwnStage {
-  float* buf;     // [2 buffers][arrays][2 blocks][P][32]
-  uint32_t mbar;  // two mbarriers, 8 bytes apart
-};
-
 
 }  // namespace umwm

@@ -61,7 +61,7 @@ __global__ void k_diag(const Params prm, const Ptrs P) {
 #pragma unroll 4
     for (int p = 0; p < NP; ++p) {
       const float cth = prm.cth[p], sth = prm.sth[p];
-      const float e = Eo[p * 32];
+      const float e = Eo[poff(p)];
       const float ek = e * kdk;
       m0 += ek;
       m2 += (f2 * e) * kdk;
@@ -113,7 +113,7 @@ __global__ void k_stokes(const Params prm, const Ptrs P) {
     const float* Eo = P.E + sidx(prm, o, 0, j);
 #pragma unroll 4
     for (int p = 0; p < NP; ++p) {
-      const float e = Eo[p * 32];
+      const float e = Eo[poff(p)];
       x += e * prm.cth[p];
       y += e * prm.sth[p];
     }
@@ -184,43 +184,71 @@ __global__ void k_screen(const Params prm, const Ptrs P) {
   screen_member<256, 256>(prm, P, blockIdx.x, s0, s2);
 }
 
-// Reference order F(om,pm,im) (o fastest) <-> the blocked device layout.
-__global__ void k_to_ref(const Params prm, const float* __restrict__ E, float* __restrict__ F, int off, int n) {
-  __shared__ float tile[32][33];
-  const int R = prm.O * prm.P;
-  const int c0 = blockIdx.x * 32, j0 = blockIdx.y * 32;
-  const int tx = threadIdx.x, ty = threadIdx.y;
-  for (int k = ty; k < 32; k += blockDim.y) {
-    const int c = c0 + k;  // column of F: c = p*O + o
-    if (c < R && j0 + tx < n) {
-      const int o = c % prm.O, p = c / prm.O;
-      tile[k][tx] = E[sidx(prm, o, p, off + j0 + tx)];
+// Reference order F(om,pm,im) (o fastest) <-> the blocked device layout, one
+// CTA per 32 wet points (from `off`, which need not start a block) and four
+// directions: reads of 16 bytes per point and level, rows of 4 om floats per
+// point on the reference's side, turned through shared memory.
+template <bool TO_REF>
+__global__ void __launch_bounds__(256) k_ref(const Params prm, float* __restrict__ E, float* __restrict__ F, int off,
+                                             int n) {
+  extern __shared__ float tile[];  // [32][4 om + 1]
+  const int O = prm.O, pitch = 4 * O + 1;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const int j0 = blockIdx.x * 32, p = blockIdx.y * 4;
+  const int cnt = min(32, n - j0);
+  auto ref_side = [&](bool out) {  // a warp per point
+    for (int i = w; i < cnt; i += nw) {
+      float* f = F + ((size_t)(j0 + i) * prm.P + p) * O;
+      for (int c = lane; c < 4 * O; c += 32) {
+        if (out) f[c] = tile[i * pitch + c];
+        else tile[i * pitch + c] = f[c];
+      }
     }
-  }
+  };
+  auto dev_side = [&](bool out) {  // a warp per level, lane = point
+    for (int o = w; o < O; o += nw) {
+      if (lane >= cnt) continue;
+      float4* e = reinterpret_cast<float4*>(E + sidx(prm, o, p, off + j0 + lane));
+      float* t = tile + lane * pitch + o;
+      if (out) {
+        *e = make_float4(t[0], t[O], t[2 * O], t[3 * O]);
+      } else {
+        const float4 v = *e;
+        t[0] = v.x; t[O] = v.y; t[2 * O] = v.z; t[3 * O] = v.w;
+      }
+    }
+  };
+  if (TO_REF) dev_side(false);
+  else ref_side(false);
   __syncthreads();
-  for (int k = ty; k < 32; k += blockDim.y) {
-    const int jrow = j0 + k, c = c0 + tx;
-    if (jrow < n && c < R) F[(size_t)jrow * R + c] = tile[tx][k];
-  }
+  if (TO_REF) ref_side(true);
+  else dev_side(true);
 }
 
-__global__ void k_from_ref(const Params prm, const float* __restrict__ F, float* __restrict__ E, int off, int n) {
-  __shared__ float tile[32][33];
-  const int R = prm.O * prm.P;
-  const int c0 = blockIdx.x * 32, j0 = blockIdx.y * 32;
-  const int tx = threadIdx.x, ty = threadIdx.y;
-  for (int k = ty; k < 32; k += blockDim.y) {
-    const int jrow = j0 + k, c = c0 + tx;
-    if (jrow < n && c < R) tile[k][tx] = F[(size_t)jrow * R + c];
+// The mss prefix (Ptrs::MSS) of blocks [b0, b0 + gridDim.x) from e: after a
+// state was set; the propagation keeps it from then on.
+__global__ void __launch_bounds__(128) k_mss(const Params prm, const Ptrs P, int b0) {
+  __shared__ float v[MAX_OM * 96];
+  const int blk = b0 + blockIdx.x, lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const int j = blk * 32 + lane;
+  for (int o = w; o < prm.O; o += nw) {
+    const float4* r = reinterpret_cast<const float4*>(P.E + sidx(prm, o, 0, j));
+    float a = 0.f, b = 0.f, c = 0.f;
+    for (int q = 0; q < prm.P / 4; ++q) {
+      const float4 e = r[q * 32];
+      const float* c2 = prm.dc2th + 4 * q;
+      const float* s2 = prm.ds2th + 4 * q;
+      a += (e.x + e.y) + (e.z + e.w);
+      b += e.x * c2[0] + e.y * c2[1] + e.z * c2[2] + e.w * c2[3];
+      c += e.x * s2[0] + e.y * s2[1] + e.z * s2[2] + e.w * s2[3];
+    }
+    const float hk = P.TAB[tidx(prm, o, T_K3DK, j)] * (0.5f * prm.dth);
+    v[o * 96 + lane] = hk * a;
+    v[o * 96 + 32 + lane] = hk * b;
+    v[o * 96 + 64 + lane] = hk * c;
   }
   __syncthreads();
-  for (int k = ty; k < 32; k += blockDim.y) {
-    const int c = c0 + k;
-    if (c < R && j0 + tx < n) {
-      const int o = c % prm.O, p = c / prm.O;
-      E[sidx(prm, o, p, off + j0 + tx)] = tile[tx][k];
-    }
-  }
+  if (w < 3) mss_prefix(prm, P, blk, w, v, 96);
 }
 
 // start of a dtg: sumt = 0 and no member done (umwm_top.F90:88)
@@ -386,14 +414,21 @@ cudaError_t launch_screen(const Params& prm, const Ptrs& P, cudaStream_t st) {
   k_screen<<<prm.nmem, 256, 0, st>>>(prm, P);
   return cudaGetLastError();
 }
-cudaError_t launch_to_ref(const Params& prm, const float* E, float* F, int off, int n, cudaStream_t st) {
-  dim3 grid((prm.O * prm.P + 31) / 32, (n + 31) / 32), block(32, 8);
-  k_to_ref<<<grid, block, 0, st>>>(prm, E, F, off, n);
+template <bool TO_REF>
+static cudaError_t launch_ref(const Params& prm, float* E, float* F, int off, int n, cudaStream_t st) {
+  if (n <= 0) return cudaSuccess;
+  const dim3 grid((n + 31) / 32, prm.P / 4);
+  k_ref<TO_REF><<<grid, 256, (size_t)32 * (4 * prm.O + 1) * sizeof(float), st>>>(prm, E, F, off, n);
   return cudaGetLastError();
 }
+cudaError_t launch_to_ref(const Params& prm, const float* E, float* F, int off, int n, cudaStream_t st) {
+  return launch_ref<true>(prm, const_cast<float*>(E), F, off, n, st);
+}
 cudaError_t launch_from_ref(const Params& prm, const float* F, float* E, int off, int n, cudaStream_t st) {
-  dim3 grid((prm.O * prm.P + 31) / 32, (n + 31) / 32), block(32, 8);
-  k_from_ref<<<grid, block, 0, st>>>(prm, F, E, off, n);
+  return launch_ref<false>(prm, E, const_cast<float*>(F), off, n, st);
+}
+cudaError_t launch_mss(const Params& prm, const Ptrs& P, int off, int padded, cudaStream_t st) {
+  k_mss<<<padded / 32, 128, 0, st>>>(prm, P, off / 32);
   return cudaGetLastError();
 }
 cudaError_t launch_begin_dtg(const Params& prm, cudaStream_t st) {

@@ -81,24 +81,29 @@ __device__ __forceinline__ void forcing_stage(const Params& prm, const Ptrs& P, 
   }
 }
 
-template <int G, int H, bool CURV>
-union PersistSmem {
-  SrcSmem<G, H, false> phys;
-  SrcSmem<G, H, true> integ;
-  AdvSmem<G, H, CURV> adv;
-  float scr[2][256];
-};
+// dynamic shared memory of the stages, one after another: the propagation's
+// level sums and rows in flight, the integration's cos(wdir - th) per warp
+template <int NP>
+static size_t persist_smem(int om) {
+  return sizeof(float) * std::max(adv_red_floats(om) + 4 * adv_ring_floats<NP>(), (size_t)4 * NP * 32);
+}
 
-template <int G, int H, bool CURV>
+template <int NP, bool CURV>
 #ifndef UMWM_PERSIST_MINB
 #define UMWM_PERSIST_MINB 4  // resident CTAs per SM (3, at 168 registers: 12.42 ms per substep against 11.71)
 #endif
 __global__ void __launch_bounds__(128, UMWM_PERSIST_MINB)
     k_persist(const Params prm, const Ptrs P, unsigned expected, unsigned long long limit_ns) {
-  __shared__ PersistSmem<G, H, CURV> sm;
+  extern __shared__ __align__(128) float dsm[];
+  __shared__ float phys_s[4 * 64], scr[2][256];
   __shared__ int ok_s;
-  constexpr int PPC = 4 * (32 / G);  // points of a spectral CTA tile
-  const int nvb = prm.Ntot / PPC;
+  __shared__ float4 dirs_s[NP / 4 * DIR_ROWS], cw[NP / 4 * 32];
+  dir_fill<NP>(prm, reinterpret_cast<float*>(dirs_s));
+  __syncthreads();
+  const uint32_t dirs = adv_smem_u32(dirs_s);
+  constexpr int NG = NP / integ_dirs<NP>();
+  const int nvb = prm.Ntot / 32;  // blocks of 32 points
+  const int warp = threadIdx.x >> 5;
   const int nb = gridDim.x;
   const int compute_rot = prm.currents;
   Global* gl = P.glob;
@@ -121,21 +126,21 @@ __global__ void __launch_bounds__(128, UMWM_PERSIST_MINB)
       for (int j = blockIdx.x * 128 + threadIdx.x; j < prm.Ntot; j += nb * 128) sice_point(prm, P, j);
       if (!bar_s(1)) return;
     }
-    for (int v = blockIdx.x; v < nvb; v += nb) source_body<G, H, false, false>(prm, P, compute_rot, v, sm.phys);
+    for (int v = blockIdx.x; v < nvb; v += nb) {
+      phys_body<NP, 0>(prm, P, compute_rot, v, dirs, cw, phys_s, nullptr, 0u);
+      __syncthreads();  // the next block reuses the maxima
+    }
     if (!bar_s(2)) return;
     if (blockIdx.x == 0) dts_body(prm, P, compute_rot, 0);
     if (!bar_s(3)) return;
-    for (int v = blockIdx.x; v < nvb; v += nb) {
-      const Ctl* ctl = prm.mem[prm.tile_mem[(v * PPC) / TILE]].ctl;
-      if (P.src_sin && (ctl->done || ctl->first) && gl->save_src)
-        source_body<G, H, true, true>(prm, P, 0, v, sm.integ);
-      else
-        source_body<G, H, true, false>(prm, P, 0, v, sm.integ);
-    }
+    for (int u = blockIdx.x * 4 + warp; u < nvb * NG; u += nb * 4) integ_body<NP>(prm, P, dirs, reinterpret_cast<float4*>(dsm) + warp * (NP / 4 * 32), u / NG, u % NG, 1);
     if (!bar_s(4)) return;
-    for (int v = blockIdx.x; v < nvb; v += nb) advect_body<G, H, CURV, false, true>(prm, P, v, sm.adv);
+    for (int v = blockIdx.x; v < nvb; v += nb) {
+      advect_body<NP, CURV, false, true>(prm, P, v, dirs, cw, dsm, dsm + adv_red_floats(prm.O));
+      __syncthreads();  // the next block reuses the sums
+    }
     if (!bar_s(5)) return;
-    for (int m = blockIdx.x; m < prm.nmem; m += nb) screen_member<256, 128>(prm, P, m, sm.scr[0], sm.scr[1]);
+    for (int m = blockIdx.x; m < prm.nmem; m += nb) screen_member<256, 128>(prm, P, m, scr[0], scr[1]);
     if (blockIdx.x == 0 && threadIdx.x == 0) gl->iters += 1;
     if (!bar_s(6)) return;
     // not_done was set by this substep's dts, two barriers ago
@@ -150,16 +155,19 @@ __global__ void k_persist_arm(Global* g) {
   g->bar_err = 0;
 }
 
-template <int G, int H, bool CURV>
+template <int NP, bool CURV>
 static cudaError_t launch_persist_t(const Params& prm, const Ptrs& P, int stall_test, cudaStream_t st) {
   int dev = 0, nsm = 0, per_sm = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_persist<G, H, CURV>, 128, 0);
+  const size_t smem = persist_smem<NP>(prm.O);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(k_persist<NP, CURV>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)persist_smem<NP>(MAX_OM));
+  if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_persist<NP, CURV>, 128, smem);
   if (e != cudaSuccess) return e;
   if (per_sm < 1) return cudaErrorLaunchOutOfResources;
-  constexpr int PPC = 4 * (32 / G);
-  const unsigned grid = (unsigned)std::max(1, std::min(nsm * per_sm, prm.Ntot / PPC));
+  const unsigned grid = (unsigned)std::max(1, std::min(nsm * per_sm, prm.Ntot / 32));
   // the barrier expects one CTA more than launched when the stall test is
   // armed: every wait then runs out after 20 ms
   const unsigned expected = grid + (stall_test ? 1u : 0u);
@@ -167,7 +175,7 @@ static cudaError_t launch_persist_t(const Params& prm, const Ptrs& P, int stall_
   k_persist_arm<<<1, 1, 0, st>>>(P.glob);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
   void* args[] = {(void*)&prm, (void*)&P, (void*)&expected, (void*)&limit_ns};
-  return cudaLaunchCooperativeKernel((const void*)k_persist<G, H, CURV>, dim3(grid), dim3(128), args, 0, st);
+  return cudaLaunchCooperativeKernel((const void*)k_persist<NP, CURV>, dim3(grid), dim3(128), args, smem, st);
 }
 
 bool persist_supported(const Params& prm) {
@@ -177,11 +185,7 @@ bool persist_supported(const Params& prm) {
 cudaError_t launch_persist(const Params& prm, const Ptrs& P, int stall_test, cudaStream_t st) {
   if (!persist_supported(prm)) return cudaErrorInvalidConfiguration;
   const bool curv = prm.curvilinear != 0;
-  if (prm.groups4)
-    return curv ? launch_persist_t<4, 9, true>(prm, P, stall_test, st)
-                : launch_persist_t<4, 9, false>(prm, P, stall_test, st);
-  return curv ? launch_persist_t<2, 18, true>(prm, P, stall_test, st)
-              : launch_persist_t<2, 18, false>(prm, P, stall_test, st);
+  return curv ? launch_persist_t<36, true>(prm, P, stall_test, st) : launch_persist_t<36, false>(prm, P, stall_test, st);
 }
 
 }  // namespace umwm

@@ -1,140 +1,140 @@
 // Source-term kernels: sin_d12, sds_d12, snl_d12, s_ice and source()
 // (umwm_source_functions.F90:16-183, umwm_physics.F90:9-86).
 //
-// Thread mapping.  The pm directions of a point are split into G groups of
-// H = pm/G consecutive directions (G = 4 when pm/4 is a supported group size,
-// else G = 2); a warp owns 32/G consecutive wet points and lane = point +
-// (32/G) * q, where group q takes directions p = qH .. qH+H-1.  Group q is the
-// base group 0 turned by q*2pi/G (a quarter turn for G = 4, a half turn for
-// G = 2), so every group runs the same code with the direction index
-// k = 0..H-1 known at compile time (every direction constant of the base
-// group is a constant-bank operand) and a per-lane rotation (ra, rb):
-// cos th = ra cos th0 - rb sin th0, sin th = rb cos th0 + ra sin th0, and
-// cos/sin 2th pick up the sign cos(2 q 2pi/G).  The groups of a point combine
-// their partial sums with log2(G) shuffles.
+// Lane = point: a warp holds 32 consecutive wet points (one block of the
+// layout) and reads four directions of all of them per instruction.
 //
-// The frequency loop walks o = 1..om in order because the mean-square-slope
-// adjustment of Sds is a prefix over o:
+// The mean-square-slope adjustment of Sds is a prefix over the levels:
 //   dummy(o,p) = dummy(o-1,p) + k3dk(o-1) * sum_pp e(o-1,pp) cth2pp(pp,p),
 //   cth2pp(pp,p) = cos^2(th(pp)-th(p)) dth
 //                = dth/2 (1 + cos2th(pp)cos2th(p) + sin2th(pp)sin2th(p)),
-// so dummy(o,.) = A + B cos2th(p) + C sin2th(p) with three running sums per
-// point (exact algebra; two multiply-adds per bin instead of pm).
-// Snl at level o needs Sds*e at o+1 and o+2, so the integration finishes
-// level o two levels after it was loaded (registers hold two levels of e and
-// Sds per direction).  Upcoming levels are prefetched into L2.
+// so dummy(o,.) = A + B cos2th(p) + C sin2th(p) with three sums per point
+// (exact algebra; two multiply-adds per bin instead of pm).  They depend on e
+// alone and are stored per level (Ptrs::MSS) by the kernel that writes e, so
+// the levels are independent of one another here.
 //
-// MODE_PHYS : per-point max |exponent argument| -> physics_time_step and the
-//             global min for dts (umwm_physics.F90:18-41); with compute_rot
-//             also the global max of the rotation rate for refraction's dtr
-//             (umwm_advection.F90:125-154).
-// MODE_INTEG: exponential integration (o <= oc), equilibrium tail (o > oc),
-//             E* = (e + ef)/2 -> ES (umwm_physics.F90:61-84); ef -> EF (= E)
-//             above the cut-off only: below it e stays and the propagation
-//             forms ef = 2 E* - e, which saves a spectrum write per substep.
+// Dts pre-pass: per-point max |exponent argument| -> physics_time_step and the
+//   global min for dts (umwm_physics.F90:18-41); with compute_rot also the
+//   global max of the rotation rate for refraction's dtr
+//   (umwm_advection.F90:125-154).  A CTA owns a block; its warps share out the
+//   prognostic levels.
+//   Bound by the SFU (two of its operations per bin) and HBM about equally.
+//   305 k points: 0.33 ms with each warp's next level staged by a bulk copy,
+//   0.36 ms loading the rows itself, 0.42 ms for the kernel this replaces (a
+//   point's directions over two lanes); 171 points: 12 us with 16 warps, 20 us
+//   with 4 (before: 26).
+// Integration: exponential integration (o <= oc), equilibrium tail (o > oc),
+//   E* = (e + ef)/2 -> ES (umwm_physics.F90:61-84); ef -> EF (= E) above the
+//   cut-off only: below it e stays and the propagation forms ef = 2 E* - e,
+//   which saves a spectrum write per substep.  A warp takes 12 (or 8)
+//   directions of a block and walks the levels downwards with the two levels
+//   above in registers (Snl); small models split the levels over several
+//   warps of the block's CTA.
+//   Bound by issue slots and latency at 15 warps per SM (128 registers).  The
+//   walk is downwards so that Snl's two levels are registers, not shared
+//   memory; a level's branch (below the cut-off, above, mixed) is taken once
+//   for the warp.  305 k points: 0.75 ms (before: 0.84); 171 points: 23 us in
+//   five chunks, 43 us in one (before: 47).
+#include <algorithm>
+
 #include "kernels.hpp"
 #include "src_body.cuh"
 
 namespace umwm {
 
-// Resident CTAs per SM the register budget of each instance is sized for
-// when no tuned value applies.
-template <int G, int H, bool INTEG>
-constexpr int default_minb() {
-  return G == 4 ? (INTEG ? 4 : 5) : (INTEG ? (UMWM_INTEG_SMEM_LAGS && H <= 18 ? UMWM_INTEG_MINB : 3) : UMWM_PHYS_MINB);
+template <int NP, int W, int MINB, int TMA = 0>
+__global__ void __launch_bounds__(W * 32, MINB) k_phys(const Params prm, const Ptrs P, int compute_rot) {
+  extern __shared__ __align__(128) float dsm[];
+  __shared__ float red[W * 64];
+  __shared__ float4 dirs[NP / 4 * DIR_ROWS], cw[NP / 4 * 32];
+  __shared__ __align__(8) unsigned long long mbar[TMA ? 2 * W : 1];
+  dir_fill<NP>(prm, reinterpret_cast<float*>(dirs));  // (phys_body's barrier)
+  phys_body<NP, TMA>(prm, P, compute_rot, blockIdx.x, adv_smem_u32(dirs), cw, red, dsm, adv_smem_u32(mbar));
 }
 
-template <int G, int H, bool INTEG, int MINB>
-__global__ void __launch_bounds__(128, MINB) k_source(const Params prm, const Ptrs P, int compute_rot) {
-  __shared__ SrcSmem<G, H, INTEG> sm;
-  if (INTEG && P.src_sin) {
-    // the last substep of a step that computes stress('ocn') or writes output
-    // keeps its source terms, and so does the model's first substep (its
-    // spectrum output)
-    const Ctl* ctl = prm.mem[prm.tile_mem[(blockIdx.x * (4 * 32 / G)) / TILE]].ctl;
-    if ((ctl->done || ctl->first) && P.glob->save_src) {
-      source_body<G, H, INTEG, true>(prm, P, compute_rot, blockIdx.x, sm);
-      return;
-    }
+template <int NP, int W, int MINB, int TMA = 0>
+static cudaError_t go_phys(const Params& prm, const Ptrs& P, int compute_rot, int warps, cudaStream_t st) {
+  const size_t smem = TMA ? (size_t)warps * 2 * NP * 32 * sizeof(float) : 0;
+  if (TMA) {
+    static std::atomic<unsigned long long> done{0};
+    const cudaError_t e =
+        allow_smem((const void*)k_phys<NP, W, MINB, TMA>, (size_t)W * 2 * NP * 32 * sizeof(float), done);
+    if (e != cudaSuccess) return e;
   }
-  source_body<G, H, INTEG, false>(prm, P, compute_rot, blockIdx.x, sm);
-}
-
-// k_source_tma: the dts pre-pass with its own e rows staged in shared memory
-// by bulk copies (OwnStage), for the two-group mapping; 5 CTAs per SM.
-template <int G, int H>
-__global__ void __launch_bounds__(128, 5) k_source_tma(const Params prm, const Ptrs P, int compute_rot) {
-  extern __shared__ __align__(128) unsigned char dsm[];
-  __shared__ __align__(8) unsigned long long mbar[2];
-  auto& sm = *reinterpret_cast<SrcSmem<G, H, false>*>(dsm);
-  constexpr size_t off = (sizeof(SrcSmem<G, H, false>) + 127) & ~size_t(127);
-  const OwnStage own{reinterpret_cast<float*>(dsm + off), adv_smem_u32(mbar)};
-  source_body<G, H, false, false, true>(prm, P, compute_rot, blockIdx.x, sm, own);
-}
-
-// Launch with the register budget of `minb` resident CTAs per SM.  The
-// 36-direction mappings (the configured workloads) have instances for the
-// budgets the autotuner tries (the integration's shared memory allows at
-// most 4 CTAs of the two-group mapping); other budgets and direction counts
-// use the default instance.
-template <int G, int H, bool INTEG>
-static void launch_src(int minb, dim3 grid, const Params& prm, const Ptrs& P, int compute_rot, cudaStream_t st) {
-  const dim3 block(128);
-#define INST(B)                                                              \
-  case B:                                                                    \
-    k_source<G, H, INTEG, B><<<grid, block, 0, st>>>(prm, P, compute_rot);   \
-    return;
-  if constexpr (G == 2 && H == 18 && INTEG) {
-    switch (minb) { INST(3) INST(4) default: break; }
-  } else if constexpr (G == 2 && H == 18) {
-    if (prm.phys_tma) {
-      const size_t smem = ((sizeof(SrcSmem<2, 18, false>) + 127) & ~size_t(127)) + (size_t)2 * 2 * prm.P * 32 * 4;
-      static const cudaError_t attr =
-          cudaFuncSetAttribute(k_source_tma<2, 18>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-      if (attr == cudaSuccess) {
-        k_source_tma<2, 18><<<grid, block, smem, st>>>(prm, P, compute_rot);
-        return;
-      }
-    }
-    switch (minb) { INST(5) INST(6) INST(7) default: break; }
-  } else if constexpr (G == 4 && H == 9) {
-    switch (minb) { INST(3) INST(4) INST(5) INST(6) default: break; }
-  }
-#undef INST
-  k_source<G, H, INTEG, default_minb<G, H, INTEG>()><<<grid, block, 0, st>>>(prm, P, compute_rot);
-}
-
-template <bool INTEG>
-static cudaError_t launch_source_t(const Params& prm, const Ptrs& P, int compute_rot, cudaStream_t st) {
-  const int minb = INTEG ? prm.minb_integ : prm.minb_phys;
-  if ((INTEG ? prm.groups4 : prm.groups4_phys) && quarter_groups(prm.P)) {
-    const dim3 grid(prm.ntiles * (TILE / 32));  // 32 points per CTA
-    switch (prm.P / 4) {
-#define CASE(X) \
-  case X: launch_src<4, X, INTEG>(minb, grid, prm, P, compute_rot, st); break;
-      CASE(4) CASE(6) CASE(8) CASE(9) CASE(12)
-#undef CASE
-      default: return cudaErrorInvalidConfiguration;
-    }
-    return cudaGetLastError();
-  }
-  const dim3 grid(prm.ntiles);  // 64 points per CTA
-  switch (prm.P / 2) {
-#define CASE(X) \
-  case X: launch_src<2, X, INTEG>(minb, grid, prm, P, compute_rot, st); break;
-    CASE(4) CASE(6) CASE(8) CASE(12) CASE(16) CASE(18) CASE(24)
-#undef CASE
-    default: return cudaErrorInvalidConfiguration;
-  }
+  k_phys<NP, W, MINB, TMA><<<prm.Ntot / 32, warps * 32, smem, st>>>(prm, P, compute_rot);
   return cudaGetLastError();
 }
 
+// prm.groups4_phys: 16 warps per block (8 where the blocks are more than one
+// per SM) instead of 4.  prm.phys_tma (36 directions): the staged form; 0: the
+// form that loads its rows itself, with prm.minb_phys the resident CTAs its
+// register budget is sized for.
+template <int NP>
+static cudaError_t launch_phys_np(const Params& prm, const Ptrs& P, int compute_rot, cudaStream_t st) {
+  if (prm.groups4_phys) return go_phys<NP, 16, 1>(prm, P, compute_rot, prm.Ntot / 32 <= prm.nsm ? 16 : 8, st);
+  if constexpr (NP == 36) {
+    if (prm.phys_tma) return go_phys<NP, 4, 5, 1>(prm, P, compute_rot, 4, st);
+    if (prm.minb_phys == 5) return go_phys<NP, 4, 5>(prm, P, compute_rot, 4, st);
+    if (prm.minb_phys == 7) return go_phys<NP, 4, 7>(prm, P, compute_rot, 4, st);
+  }
+  return go_phys<NP, 4, 6>(prm, P, compute_rot, 4, st);
+}
+
+// The integration: NG direction groups x nc level chunks of one block per CTA.
+template <int NP, int WMAX, int MINB>
+__global__ void __launch_bounds__(WMAX * 32, MINB) k_integ(const Params prm, const Ptrs P, int nc) {
+  // cos(wdir - th) per level chunk: the chunks' warps then need no barrier
+  constexpr int NG = NP / integ_dirs<NP>(), NC = WMAX / NG;
+  __shared__ float4 dirs[NP / 4 * DIR_ROWS], cw[NC * NP / 4 * 32];
+  dir_fill<NP>(prm, reinterpret_cast<float*>(dirs));
+  __syncthreads();
+  const int w = threadIdx.x >> 5;
+  integ_body<NP>(prm, P, adv_smem_u32(dirs), cw + (w / NG) * (NP / 4 * 32), blockIdx.x, w, nc);
+}
+
+template <int NP, int WMAX, int MINB>
+static cudaError_t go_integ(const Params& prm, const Ptrs& P, int nc, cudaStream_t st) {
+  k_integ<NP, WMAX, MINB><<<prm.Ntot / 32, 32 * nc * (NP / integ_dirs<NP>()), 0, st>>>(prm, P, nc);
+  return cudaGetLastError();
+}
+
+// prm.groups4: the levels of a block in several chunks (small models: the
+// walk over all levels is the time of the kernel there).  Else the register
+// budget of 15 warps per SM (128 registers, no spills), or of 18 where the
+// blocks then fit one wave instead of two.  prm.minb_integ 3, 5: 12, 18 warps.
+template <int NP>
+static cudaError_t launch_integ_np(const Params& prm, const Ptrs& P, cudaStream_t st) {
+  constexpr int NG = NP / integ_dirs<NP>(), C15 = std::max(1, 15 / NG), C18 = std::max(1, 18 / NG);
+  const int blocks = prm.Ntot / 32;
+  if (prm.groups4) {
+    const int nc = std::min(blocks <= 2 * prm.nsm ? 16 / NG : 2, prm.O / 4);
+    if (nc > 1) return go_integ<NP, 16, 1>(prm, P, nc, st);
+  }
+  if (NP == 36 && prm.minb_integ == 3) return go_integ<NP, NG, 4>(prm, P, 1, st);
+  if (prm.minb_integ == 5 || (blocks > C15 * prm.nsm && blocks <= C18 * prm.nsm))
+    return go_integ<NP, NG, C18>(prm, P, 1, st);
+  return go_integ<NP, NG, C15>(prm, P, 1, st);
+}
+
+#define UMWM_ALL_NP(F, ...)                      \
+  switch (prm.P) {                               \
+    case 8: return F<8>(__VA_ARGS__);            \
+    case 12: return F<12>(__VA_ARGS__);          \
+    case 16: return F<16>(__VA_ARGS__);          \
+    case 24: return F<24>(__VA_ARGS__);          \
+    case 32: return F<32>(__VA_ARGS__);          \
+    case 36: return F<36>(__VA_ARGS__);          \
+    case 48: return F<48>(__VA_ARGS__);          \
+    default: return cudaErrorInvalidConfiguration; \
+  }
+
 cudaError_t launch_source_phys(const Params& prm, const Ptrs& P, int compute_rot, cudaStream_t st) {
-  return launch_source_t<false>(prm, P, compute_rot, st);
+  UMWM_ALL_NP(launch_phys_np, prm, P, compute_rot, st)
 }
 cudaError_t launch_source_integ(const Params& prm, const Ptrs& P, cudaStream_t st) {
-  return launch_source_t<true>(prm, P, 0, st);
+  UMWM_ALL_NP(launch_integ_np, prm, P, st)
 }
+
 bool supported_pm(int pm) {
   const int h = pm / 2;
   return pm % 4 == 0 && (h == 4 || h == 6 || h == 8 || h == 12 || h == 16 || h == 18 || h == 24);

@@ -100,12 +100,12 @@ __global__ void __launch_bounds__(256) k_features(const Params prm, const Ptrs P
     const int nl = min(FLC, prm.O - c0);  // levels of this chunk
     const int o = c0 + warp;
     if (warp < nl) {
-      const float* Er = ok ? P.E + sidx(prm, o, 0, j) : nullptr;  // direction p at Er[p * 32]
+      const float* Er = ok ? P.E + sidx(prm, o, 0, j) : nullptr;  // direction p at Er[poff(p)]
       int pr = s == 0 ? 0 : NP - s;                                  // rotated column of p = 0
       for (int p0 = 0; p0 < NP; p0 += UNR) {
         float ev[UNR];
 #pragma unroll
-        for (int u = 0; u < UNR; ++u) ev[u] = (ok && p0 + u < NP) ? __ldg(Er + (p0 + u) * 32) : 0.f;
+        for (int u = 0; u < UNR; ++u) ev[u] = (ok && p0 + u < NP) ? __ldg(Er + poff(p0 + u)) : 0.f;
 #pragma unroll
         for (int u = 0; u < UNR; ++u) {
           if (p0 + u >= NP) break;

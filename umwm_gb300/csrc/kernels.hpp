@@ -2,9 +2,22 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <atomic>
+
 #include "dev.cuh"
 
 namespace umwm {
+
+// Lets kernel f take `bytes` of dynamic shared memory on the current device
+// (once per kernel and device; done: the devices it has been set on).
+inline cudaError_t allow_smem(const void* f, size_t bytes, std::atomic<unsigned long long>& done) {
+  int d = 0;
+  cudaError_t e = cudaGetDevice(&d);
+  if (e != cudaSuccess || (d < 64 && (done.load(std::memory_order_relaxed) >> d & 1))) return e;
+  e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  if (e == cudaSuccess && d < 64) done.fetch_or(1ull << d, std::memory_order_relaxed);
+  return e;
+}
 
 bool supported_pm(int pm);
 cudaError_t launch_prep(const Params& prm, const Ptrs& P, int compute_rot, int max_nm, cudaStream_t st);
@@ -18,6 +31,8 @@ cudaError_t launch_stokes(const Params& prm, const Ptrs& P, cudaStream_t st);
 cudaError_t launch_screen(const Params& prm, const Ptrs& P, cudaStream_t st);
 cudaError_t launch_to_ref(const Params& prm, const float* E, float* F, int off, int n, cudaStream_t st);
 cudaError_t launch_from_ref(const Params& prm, const float* F, float* E, int off, int n, cudaStream_t st);
+// the mss prefix of the points [off, off + padded) (whole blocks) from e
+cudaError_t launch_mss(const Params& prm, const Ptrs& P, int off, int padded, cudaStream_t st);
 cudaError_t launch_begin_dtg(const Params& prm, cudaStream_t st);
 cudaError_t launch_stress_ocn(const Params& prm, const Ptrs& P, cudaStream_t st);
 cudaError_t launch_loop_arm(Global* g, int budget, cudaStream_t st);

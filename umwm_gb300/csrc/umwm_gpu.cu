@@ -96,7 +96,7 @@ struct MemberHost {
 // Online autotuner of the three spectral kernels' launch configuration.
 //
 // Each kernel (dts pre-pass, integration, propagation) has a candidate list
-// of (direction mapping, resident CTAs per SM, prefetch distance).  While the
+// of (split of the levels, resident CTAs per SM, prefetch distance).  While the
 // tuner is active the inner loop runs host-driven and substep s launches each
 // kernel with its candidate s mod n (round-robin, `reps` times each), timed
 // with CUDA events on the model's stream; once a kernel has all its samples
@@ -104,13 +104,12 @@ struct MemberHost {
 // adds time, and the interleaving spreads drift over all candidates).  The
 // tuner measures the
 // model's real substeps, so tuning costs no extra work.  Register budgets and
-// prefetch distances do not change any result (mode 1); the direction mapping
-// changes the summation order of the partial sums (mode 2, results differ by
-// rounding: both mappings meet the parity bars).  Choices are cached per
+// prefetch distances do not change any result, nor does the split of the
+// levels over more warps (mode 2).  Choices are cached per
 // domain signature for the life of the process.
 struct TuneCand {
-  int g4, minb, pf;  // quarter-turn groups, CTAs per SM (0: default instance), levels prefetched
-  int tma = 0;       // own rows staged by bulk copies (propagation 1: E* and e, 2: E*; pre-pass 1: e)
+  int g4, minb, pf;  // levels over more warps, CTAs per SM (0: default instance), levels prefetched
+  int tma = 0;       // rows staged by bulk copies (pre-pass; the propagation stages its rows in every form)
 };
 struct KernelTune {
   std::vector<TuneCand> cands;
@@ -305,9 +304,8 @@ void tune_set(Params& p, int k, const TuneCand& c) {
   else { p.adv_groups4 = c.g4; p.minb_adv = c.minb; p.pf_adv = c.pf; p.adv_tma = c.tma; }
 }
 
-// Candidate lists.  Register budgets have kernel instances only for the
-// 36-direction mappings (the integration's two-group shared memory allows at
-// most 4 CTAs; the propagation's tuned instances are for plain grids).
+// Candidate lists.  Budgets have kernel instances only for 36 directions and
+// the 4-warp mapping (elsewhere a budget runs the default instance).
 void tune_start(Model& M, int mode) {
   Tuner& T = M.tune;
   T.mode = mode;
@@ -343,12 +341,11 @@ void tune_start(Model& M, int mode) {
       }
       for (int mb : minbs)
         for (int pf : pfs) K.cands.push_back({g4, mb, pf, 0});
-      // the propagation (3 CTAs per SM) and the dts pre-pass (5) with their
-      // own rows staged by bulk copies
+      // and with the rows staged (for the propagation the forms above again)
       if (k == TK_ADVECT && d36 && !p.curvilinear && !g4)
         for (int pf : pfs) {
-          K.cands.push_back({0, 3, pf, 1});  // E* and e staged
-          K.cands.push_back({0, 4, pf, 2});  // E* staged
+          K.cands.push_back({0, 3, pf, 1});
+          K.cands.push_back({0, 4, pf, 2});
         }
       if (k == TK_PHYS && d36 && !g4)
         for (int pf : {1, 2}) K.cands.push_back({0, 5, pf, 1});
@@ -433,34 +430,40 @@ cudaError_t tuned(Model& M, int tk, int kname, F&& launch) {
   return e;
 }
 
-// per-(o,i) tables in the blocked device layout [o][j/32][t][32], one member
-// at a time (host memory of one member).  A member's ghost point holds the
-// ghost values of cp0/cg0; padding points get finite throw-away values (k = 1)
-// so that idle lanes stay finite.  Members start on a tile boundary, so for
-// each o a member's blocks are one contiguous range.
+// per-(o,i) tables in the blocked device layout [j/32][o][t][32], one member
+// at a time.  A member's ghost point holds the ghost values of cp0/cg0;
+// padding points get finite throw-away values (k = 1) so that idle lanes stay
+// finite.  Members start on a tile boundary, so a member's blocks are one
+// contiguous range.
 int upload_tables(Model& M, const MemberHost& mh) {
   const Params& prm = M.prm;
   const int O = prm.O;
   const HostModel& H = mh.H;
   const std::vector<float>* src[T_COUNT] = {};
   src[T_K] = &H.k, src[T_CP0] = &H.cp0, src[T_CG0] = &H.cg0, src[T_LOGL2Z] = &H.logl2overz;
-  src[T_FKOVG] = &H.fkovg, src[T_KDK] = &H.kdk, src[T_K4] = &H.k4, src[T_K3DK] = &H.k3dk;
-  src[T_COTHKD] = &H.cothkd, src[T_SBF] = &H.sbf, src[T_SDV] = &H.sdv, src[T_BF1R] = &H.bf1r;
-  src[T_BF2R] = &H.bf2r;
-  const size_t per_o = (size_t)mh.padded * T_COUNT;  // floats of one level of this member
-  std::vector<float> T(per_o);
-  for (int o = 1; o <= O; ++o) {
-    for (int t = 0; t < T_COUNT; ++t) {
-      const bool ghost = (t == T_CP0 || t == T_CG0);
-      for (int j = 0; j < mh.padded; ++j) {
-        float v;
-        if (j < mh.N) v = (*src[t])[H.oi(o, j + 1)];
-        else if (ghost) v = (*src[t])[H.oi(o, 0)];
-        else v = (t == T_K || t == T_K4 || t == T_KDK || t == T_COTHKD) ? 1.f : 0.f;
-        T[((size_t)(j >> 5) * T_COUNT + t) * 32 + (j & 31)] = v;
-      }
-    }
-    CU(cudaMemcpy(M.TAB + tidx(prm, o - 1, 0, mh.off), T.data(), per_o * 4, cudaMemcpyHostToDevice));
+  src[T_KDK] = &H.kdk, src[T_K3DK] = &H.k3dk, src[T_FKOVG] = &H.fkovg, src[T_COTHKD] = &H.cothkd, src[T_SBF] = &H.sbf, src[T_SDV] = &H.sdv;
+  src[T_BF1R] = &H.bf1r, src[T_BF2R] = &H.bf2r;
+  // a few thousand blocks at a time
+  const int nblk = mh.padded / 32, chunk = std::min(nblk, 2048);
+  const size_t per_blk = (size_t)O * T_COUNT * 32;
+  std::vector<float> T(per_blk * chunk);
+  for (int b0 = 0; b0 < nblk; b0 += chunk) {
+    const int nb = std::min(chunk, nblk - b0);
+    for (int b = 0; b < nb; ++b)
+      for (int o = 1; o <= O; ++o)
+        for (int t = 0; t < T_COUNT; ++t) {
+          const bool ghost = (t == T_CP0 || t == T_CG0);
+          float* out = &T[b * per_blk + ((size_t)(o - 1) * T_COUNT + t) * 32];
+          for (int l = 0; l < 32; ++l) {
+            const int j = (b0 + b) * 32 + l;
+            float v;
+            if (j < mh.N) v = (*src[t])[H.oi(o, j + 1)];
+            else if (ghost) v = (*src[t])[H.oi(o, 0)];
+            else v = (t == T_K || t == T_KDK || t == T_COTHKD) ? 1.f : 0.f;
+            out[l] = v;
+          }
+        }
+    CU(cudaMemcpy(M.TAB + tidx(prm, 0, 0, mh.off + b0 * 32), T.data(), per_blk * nb * 4, cudaMemcpyHostToDevice));
   }
   return UMWM_OK;
 }
@@ -625,8 +628,8 @@ int setup_params(Model& M) {
     p.ice_possible |= (mh.H.seaice || (mh.H.fice0 > mh.H.fice_lth));
   }
   for (int o = 0; o < H.om; ++o) { p.f[o] = H.f[o]; p.dom[o] = H.dom[o]; }
-  // the two-group flux of pm % 4 == 0 grids takes one upwind term per slot
-  // pair (adv_body.cuh): the grid th(p) = (p - (pm + 1) / 2) dth gives the
+  // the propagation takes one upwind side per direction and axis from the
+  // direction's index (adv_body.cuh): the grid th(p) = (p - (pm + 1) / 2) dth gives the
   // first pm/2 directions sin th < 0 and cos th < 0 exactly below pm/4
   p.swsign = H.pm % 4 == 0;
   for (int q = 0; q < H.pm / 2; ++q)
@@ -634,11 +637,6 @@ int setup_params(Model& M) {
   if (H.pm % 4 == 0 && !p.swsign) return fail(UMWM_ERR_NAMELIST, "direction grid without the expected signs");
   for (int q = 0; q < H.pm; ++q) {
     p.th[q] = H.th[q]; p.cth[q] = H.cth[q]; p.sth[q] = H.sth[q];
-    p.cthp[q] = std::max(H.cth[q], 0.f); p.cthm[q] = std::min(H.cth[q], 0.f);
-    const int q1 = (q + 1) % H.pm;
-    p.shs[q] = 0.5f * (H.sth[q] + H.sth[q1]);
-    p.chs[q] = 0.5f * (H.cth[q] + H.cth[q1]);
-    p.sthp[q] = std::max(H.sth[q], 0.f); p.sthm[q] = std::min(H.sth[q], 0.f);
     p.c2th[q] = (float)std::cos(2.0 * (double)H.th[q]);
     p.s2th[q] = (float)std::sin(2.0 * (double)H.th[q]);
   }
@@ -647,16 +645,12 @@ int setup_params(Model& M) {
   p.minb_phys = p.minb_integ = p.minb_adv = 0;
   p.count_cut = 0;
   p.adv_tma = 0;
-  p.phys_tma = 0;
+  p.phys_tma = 1;
   p.pf_phys = UMWM_PF_DIST_PHYS;
   p.pf_integ = UMWM_PF_DIST_INTEG;
   p.pf_adv = UMWM_PF_DIST_ADV;
   return UMWM_OK;
 }
-
-#ifndef UMWM_AUTO_G4_TILES
-#define UMWM_AUTO_G4_TILES 3
-#endif
 
 int init_device(Model& M) {
   int rc = setup_params(M);
@@ -665,17 +659,30 @@ int init_device(Model& M) {
   const int ldN = p.ldN;
   const size_t spec = (size_t)p.O * p.P * ldN;
   if (g_device >= 0) CU(cudaSetDevice(g_device));
-  // Small domains: with fewer than UMWM_AUTO_G4_TILES 64-point tiles per SM
-  // the half-turn mapping leaves SMs idle, and four quarter-turn groups (32
-  // points per CTA) double the CTAs: measured 1.4x at 9.6 k wet points,
-  // 1.3x at 17.7 k, even at 31 k (3.2 tiles per SM), 0.95x at 71 k.  The
-  // options direction_groups / advect_groups override this.
+  // Small domains: with at most one 64-point tile (two blocks) per SM the
+  // kernels' time is the walk of a block's levels, so more warps share them
+  // (options direction_groups / advect_groups 4).
   {
     int dev = 0, nsm = 0;
     CU(cudaGetDevice(&dev));
     CU(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-    if (quarter_groups(p.P) && (long)p.ntiles < (long)UMWM_AUTO_G4_TILES * nsm)
-      p.groups4 = p.groups4_phys = p.adv_groups4 = 1;
+    p.nsm = nsm;
+    if (quarter_groups(p.P) && p.ntiles <= nsm) p.groups4 = p.groups4_phys = p.adv_groups4 = 1;
+    // the direction constants: quarter turns on domains of under 192 points
+    // per SM, half turns on larger ones
+    const int turns = quarter_groups(p.P) && p.ntiles < 3 * nsm ? 4 : 2, n = p.P / turns;
+    for (int q = 0; q < p.P; ++q) {
+      const int g = (q / n) * (4 / turns);  // quarter turns from direction q % n
+      const float c = p.cth[q % n], s = p.sth[q % n], c2 = p.c2th[q % n], s2 = p.s2th[q % n];
+      p.dcth[q] = g == 0 ? c : g == 1 ? -s : g == 2 ? -c : s;
+      p.dsth[q] = g == 0 ? s : g == 1 ? c : g == 2 ? -s : -c;
+      p.dc2th[q] = g & 1 ? -c2 : c2;
+      p.ds2th[q] = g & 1 ? -s2 : s2;
+    }
+    for (int q = 0; q < p.P; ++q) {
+      p.shs[q] = 0.5f * (p.dsth[q] + p.dsth[(q + 1) % p.P]);
+      p.chs[q] = 0.5f * (p.dcth[q] + p.dcth[(q + 1) % p.P]);
+    }
   }
   M.dev.reset(new Dev());
   Dev& D = *M.dev;
@@ -692,6 +699,7 @@ int init_device(Model& M) {
   P.TAB = M.TAB;
   for (const MemberHost& mh : M.mem)
     if ((rc = upload_tables(M, mh))) return rc;
+  CU(D.alloc(&P.MSS, (size_t)p.O * 3 * ldN, true));
   // per-point arrays in the common index space
   auto upload_i = [&](const int** dst, std::vector<int>(HostModel::*field), bool aliased) -> int {
     std::vector<int> h(ldN, 0);
@@ -813,6 +821,7 @@ int init_device(Model& M) {
   const float tiny = std::numeric_limits<float>::min();
   CU(launch_fill(M.E, spec, tiny, M.st));
   CU(launch_fill(M.ES, spec, tiny, M.st));
+  CU(launch_mss(p, P, 0, ldN, M.st));
 
   // input_nc(starttimestr), umwm_top.F90:25, and init's first guess of the
   // drag and friction velocity, umwm_init.F90:1350-1365
@@ -861,6 +870,7 @@ int set_state_member(Model& M, int m, const float* F, const float* ust) {
     CU(cudaMalloc(&tmp, n * 4));
     cudaError_t e = cudaMemcpy(tmp, F, n * 4, cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = launch_from_ref(p, tmp, M.E, mh.off, mh.N, M.st);
+    if (e == cudaSuccess) e = launch_mss(p, M.P, mh.off, mh.padded, M.st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(M.st);
     cudaFree(tmp);
     CU(e);
@@ -1221,7 +1231,7 @@ int output_spectrum(Model& M, int64_t t) {
   const HostModel& H = mh.H;
   const int O = p.O, NPd = p.P;
   const size_t nb = (size_t)O * NPd;
-  const size_t tstride = (size_t)p.NB * T_COUNT * 32;
+  const size_t tstride = (size_t)T_COUNT * 32;
   CU(cudaStreamSynchronize(M.st));
   float* tmp = nullptr;
   CU(cudaMalloc(&tmp, nb * 4));
@@ -2035,18 +2045,15 @@ int umwm_gpu_get_field(const char* name, float* out, long n) {
     return UMWM_OK;
   }
   // tables (om, im) with o fastest; cp0/cg0 (om, 0:im)
-  static const std::pair<const char*, int> tabs[] = {
-      {"k", T_K}, {"cp0", T_CP0}, {"cg0", T_CG0}, {"logl2overz", T_LOGL2Z}, {"fkovg", T_FKOVG}, {"k4", T_K4},
-      {"k3dk", T_K3DK}, {"kdk", T_KDK}, {"cothkd", T_COTHKD}, {"sbf", T_SBF}, {"sdv", T_SDV},
-      {"bf1_renorm", T_BF1R}, {"bf2_renorm", T_BF2R}};
+  static const std::pair<const char*, std::vector<float> HostModel::*> tabs[] = {
+      {"k", &HostModel::k}, {"cp0", &HostModel::cp0}, {"cg0", &HostModel::cg0},
+      {"logl2overz", &HostModel::logl2overz}, {"fkovg", &HostModel::fkovg}, {"k4", &HostModel::k4},
+      {"k3dk", &HostModel::k3dk}, {"kdk", &HostModel::kdk}, {"cothkd", &HostModel::cothkd}, {"sbf", &HostModel::sbf},
+      {"sdv", &HostModel::sdv}, {"bf1_renorm", &HostModel::bf1r}, {"bf2_renorm", &HostModel::bf2r}};
   for (auto& t : tabs)
     if (s == t.first) {
-      const bool ghost = (t.second == T_CP0 || t.second == T_CG0);
-      const std::vector<float>& src = t.second == T_K ? H.k : t.second == T_CP0 ? H.cp0 : t.second == T_CG0 ? H.cg0
-          : t.second == T_LOGL2Z ? H.logl2overz : t.second == T_FKOVG ? H.fkovg : t.second == T_K4 ? H.k4
-          : t.second == T_K3DK ? H.k3dk : t.second == T_KDK ? H.kdk : t.second == T_COTHKD ? H.cothkd
-          : t.second == T_SBF ? H.sbf : t.second == T_SDV ? H.sdv : t.second == T_BF1R ? H.bf1r : H.bf2r;
-      const int lo = ghost ? 0 : 1;
+      const std::vector<float>& src = H.*t.second;
+      const int lo = s == "cp0" || s == "cg0" ? 0 : 1;  // cp0, cg0 with the ghost point first
       if (need((long)O * (N - lo + 1))) return UMWM_ERR_ARG;
       for (int i = lo; i <= N; ++i)
         for (int o = 1; o <= O; ++o) out[(size_t)(i - lo) * O + (o - 1)] = src[H.oi(o, i)];
@@ -2232,8 +2239,7 @@ int umwm_gpu_set_option(const char* name, double value) {
       return UMWM_OK;
     }
   }
-  if (s == "advect_tma" || s == "phys_tma") {  // own rows staged by bulk copies (two groups, pm 36)
-    // advect_tma 1: E* and e rows, 2: E* rows only; phys_tma 1: e rows
+  if (s == "advect_tma" || s == "phys_tma") {  // phys_tma: rows staged by bulk copies (4 warps, pm 36)
     (s == "advect_tma" ? M->prm.adv_tma : M->prm.phys_tma) =
         s == "advect_tma" ? std::max(0, std::min(2, (int)value)) : (value != 0 ? 1 : 0);
     drop_graph(*M);
