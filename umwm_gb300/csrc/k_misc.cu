@@ -29,64 +29,140 @@ __global__ void k_dts(const Params prm, const Ptrs P, int compute_rot, int first
   dts_body(prm, P, compute_rot, first);
 }
 
-// s_ice: significant wave height where fice > fice_lth and the attenuation
-// factor C1*Hs (Hs < 3 m) or C1*3 (umwm_source_functions.F90:108-153).
-__global__ void k_sice(const Params prm, const Ptrs P) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j < prm.Ntot) sice_point(prm, P, j);
+// The once-per-interval kernels below and the sea-ice wave height share one
+// mapping: a CTA owns a block of 32 points (lane = point), its MW warps take
+// every MW-th frequency level and read four directions of 32 points per
+// access, and the warps' partial sums meet in shared memory.  One thread per
+// point walked 1332 bins in a chain of dependent loads: 94 us at 171 points
+// and 543 us at 305 k for the diagnostics, 270 and 1140 us for the Stokes
+// drift, 74 us per substep at 13 k points for the sea-ice wave height.  So
+// split: 18 and 503 us, 26 and 493 us, and 23 us (small models wait on the
+// levels' chain; at 305 k points the 1.6 GB spectrum is read at 3.2 TB/s, the
+// rest being the level sums' instructions).
+constexpr int MW = 8;
+
+struct BlockPoint {
+  int j, lane, w;
+  bool valid;
+};
+// false (for the whole CTA): a block of padding
+__device__ __forceinline__ bool block_point(const Member& Mb, BlockPoint& b) {
+  b.lane = threadIdx.x & 31;
+  b.w = threadIdx.x >> 5;
+  b.j = blockIdx.x * 32 + b.lane;
+  b.valid = b.j < Mb.ghost;
+  return blockIdx.x * 32 < Mb.ghost;
+}
+// cos th and sin th, four directions each, [pm/4][2] (then a CTA barrier)
+__device__ __forceinline__ void fill_cs(const Params& prm, float* cs) {
+  for (int p = threadIdx.x; p < prm.P; p += blockDim.x) {
+    cs[(p >> 2) * 8 + (p & 3)] = prm.cth[p];
+    cs[(p >> 2) * 8 + 4 + (p & 3)] = prm.sth[p];
+  }
 }
 
-// diag, umwm_physics.F90:89-205, one thread per wet point.  The bins are
-// visited frequency by frequency (the level's table rows read once), so the
-// sums run in another order than the reference's direction-outer loops; the
-// peak keeps the reference's choice among equal values, the first in its
-// (o fastest, p slowest) order.
-__global__ void k_diag(const Params prm, const Ptrs P) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= prm.Ntot) return;
-  const Member& Mb = prm.mem[prm.tile_mem[j / TILE]];
-  if (j >= Mb.ghost) return;
-  const int ja = apt(Mb, j);
-  const int O = prm.O, NP = prm.P, oc = P.oc[j];
-  const float* E = P.E;
-  auto tab = [&](int t, int o) { return P.TAB[tidx(prm, o, t, j)]; };
-  float m0 = 0.f, m2 = 0.f, m2k = 0.f, mx = 0.f, my = 0.f, cxx = 0.f, cxy = 0.f, cyy = 0.f, xc = 0.f, yc = 0.f;
+// s_ice: significant wave height where fice > fice_lth and the attenuation
+// factor C1*Hs (Hs < 3 m) or C1*3 (umwm_source_functions.F90:108-153).
+__global__ void __launch_bounds__(MW * 32) k_sice(const Params prm, const Ptrs P) {
+  __shared__ float part[MW][32];
+  const Member& M = prm.mem[prm.tile_mem[(blockIdx.x * 32) / TILE]];
+  BlockPoint b;
+  if (M.ctl->done || !block_point(M, b)) return;
+  const bool ice = b.valid && P.fice[apt(M, b.valid ? b.j : M.ghost)] > prm.fice_lth;
+  float h = 0.f;
+  if (__any_sync(0xffffffffu, ice)) h = sice_levels(prm, P, b.j, b.w, MW);
+  part[b.w][b.lane] = h;
+  __syncthreads();
+  if (b.w != 0 || !b.valid) return;
+  h = 0.f;
+  for (int i = 0; i < MW; ++i) h += part[i][b.lane];
+  P.sice_v[b.j] = ice ? sice_factor(prm, h) : 0.f;
+}
+
+// diag, umwm_physics.F90:89-205.  A level's direction sums are formed first
+// and weighted by its table rows, so the sums run in another order than the
+// reference's direction-outer loops; the peak keeps the reference's choice
+// among equal values, the first in its (o fastest, p slowest) order.
+__global__ void __launch_bounds__(MW * 32) k_diag(const Params prm, const Ptrs P) {
+  enum { M0, M2, M2K, XC, YC, MX, MY, CXX, CXY, CYY, NS };
+  __shared__ float part[MW][NS][32], pbest[MW][32];
+  __shared__ int ppeak[MW][32];  // o * MAX_PM + p
+  __shared__ float4 cs[MAX_PM / 2];
+  fill_cs(prm, reinterpret_cast<float*>(cs));
+  __syncthreads();
+  const Member& Mb = prm.mem[prm.tile_mem[(blockIdx.x * 32) / TILE]];
+  BlockPoint b;
+  if (!block_point(Mb, b)) return;
+  const int j = b.j, lane = b.lane, w = b.w, O = prm.O, NQ = prm.P / 4;
+  const int oc = b.valid ? P.oc[j] : 0;
+  float sum[NS];
+#pragma unroll
+  for (int i = 0; i < NS; ++i) sum[i] = 0.f;
   float best = -1.f;
   int op = 0, pp = 0;
-  for (int o = 0; o < O; ++o) {
-    const float kdk = tab(T_KDK, o), k3dk = tab(T_K3DK, o), f2 = prm.f[o] * prm.f[o];
-    const bool pr = o < oc;
-    const float icp = pr ? 1.f / tab(T_CP0, o) : 0.f, cg = pr ? tab(T_CG0, o) : 0.f;
-    const float* Eo = E + sidx(prm, o, 0, j);
-#pragma unroll 4
-    for (int p = 0; p < NP; ++p) {
-      const float cth = prm.cth[p], sth = prm.sth[p];
-      const float e = Eo[poff(p)];
-      const float ek = e * kdk;
-      m0 += ek;
-      m2 += (f2 * e) * kdk;
-      m2k += e * k3dk;
-      xc += ek * cth; yc += ek * sth;
-      if (ek > best || (ek == best && p < pp)) { best = ek; op = o; pp = p; }
-      if (pr) {
-        const float ekc = ek * icp;
-        mx += ekc * cth; my += ekc * sth;
-        cxx += cg * ekc * (cth * cth); cxy += cg * ekc * cth * sth; cyy += cg * ekc * (sth * sth);
+  for (int o = w; o < O; o += MW) {
+    const float* T = P.TAB + tidx(prm, o, 0, j);
+    const float kdk = T[T_KDK * 32], k3dk = T[T_K3DK * 32], f2_ = prm.f[o] * prm.f[o];
+    const float4* r = reinterpret_cast<const float4*>(P.E + sidx(prm, o, 0, j));
+    float s0 = 0.f, sc = 0.f, ss = 0.f, scc = 0.f, scs = 0.f, sss = 0.f;
+#pragma unroll 3
+    for (int q = 0; q < NQ; ++q) {
+      const float4 e4 = r[q * 32], c4 = cs[2 * q], n4 = cs[2 * q + 1];
+      const float e[4] = {e4.x, e4.y, e4.z, e4.w}, c[4] = {c4.x, c4.y, c4.z, c4.w}, n[4] = {n4.x, n4.y, n4.z, n4.w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float ec = e[i] * c[i], es = e[i] * n[i];
+        s0 += e[i];
+        sc += ec;
+        ss += es;
+        scc = fmaf(ec, c[i], scc);
+        scs = fmaf(ec, n[i], scs);
+        sss = fmaf(es, n[i], sss);
+        const float ek = e[i] * kdk;
+        const int p = 4 * q + i;
+        if (ek > best || (ek == best && p < pp)) { best = ek; op = o; pp = p; }
       }
     }
+    sum[M0] = fmaf(s0, kdk, sum[M0]);
+    sum[M2] = fmaf(f2_ * s0, kdk, sum[M2]);
+    sum[M2K] = fmaf(s0, k3dk, sum[M2K]);
+    sum[XC] = fmaf(sc, kdk, sum[XC]);
+    sum[YC] = fmaf(ss, kdk, sum[YC]);
+    if (o < oc) {
+      const float ki = kdk / T[T_CP0 * 32], kg = ki * T[T_CG0 * 32];
+      sum[MX] = fmaf(sc, ki, sum[MX]);
+      sum[MY] = fmaf(ss, ki, sum[MY]);
+      sum[CXX] = fmaf(scc, kg, sum[CXX]);
+      sum[CXY] = fmaf(scs, kg, sum[CXY]);
+      sum[CYY] = fmaf(sss, kg, sum[CYY]);
+    }
   }
-  const float rw = P.rhow[ja] * prm.dthg;
-  P.mwp[j] = sqrtf(m0 / (m2 + FLT_MIN));
-  P.momx[j] = mx * rw; P.momy[j] = my * rw;
-  P.cgmxx[j] = cxx * rw; P.cgmxy[j] = cxy * rw; P.cgmyy[j] = cyy * rw;
+#pragma unroll
+  for (int i = 0; i < NS; ++i) part[w][i][lane] = sum[i];
+  pbest[w][lane] = best;
+  ppeak[w][lane] = op * MAX_PM + pp;
+  __syncthreads();
+  if (w != 0 || !b.valid) return;
+  for (int v = 1; v < MW; ++v) {
+#pragma unroll
+    for (int i = 0; i < NS; ++i) sum[i] += part[v][i][lane];
+    const float bv = pbest[v][lane];
+    const int ov = ppeak[v][lane] / MAX_PM, pv = ppeak[v][lane] % MAX_PM;
+    if (bv > best || (bv == best && (pv < pp || (pv == pp && ov < op)))) { best = bv; op = ov; pp = pv; }
+  }
+  const int ja = apt(Mb, j);
+  const float rw = P.rhow[ja] * prm.dthg, m0 = sum[M0], m2k = sum[M2K];
+  P.mwp[j] = sqrtf(m0 / (sum[M2] + FLT_MIN));
+  P.momx[j] = sum[MX] * rw; P.momy[j] = sum[MY] * rw;
+  P.cgmxx[j] = sum[CXX] * rw; P.cgmxy[j] = sum[CXY] * rw; P.cgmyy[j] = sum[CYY] * rw;
   P.ht[j] = 4.f * sqrtf(m0 * prm.dth);
-  P.mwd[j] = atan2f(yc, xc);
+  P.mwd[j] = atan2f(sum[YC], sum[XC]);
   P.mss[j] = m2k * prm.dth;
   P.mwl[j] = 2.f * 3.14159274f * sqrtf(m0 / (m2k + FLT_MIN));
   P.dwd[j] = prm.th[pp];
-  P.dwl[j] = 2.f * 3.14159274f / tab(T_K, op);
+  P.dwl[j] = 2.f * 3.14159274f / P.TAB[tidx(prm, op, T_K, j)];
   P.dwp[j] = 1.f / prm.f[op];
-  const float c0 = tab(T_CP0, op), g0 = tab(T_CG0, op);
+  const float c0 = P.TAB[tidx(prm, op, T_CP0, j)], g0 = P.TAB[tidx(prm, op, T_CG0, j)];
   P.dcp0[j] = c0; P.dcg0[j] = g0;
   const float uc = P.uc[ja], vc = P.vc[ja];
   P.dcp[j] = c0 + uc * prm.cth[pp] + vc * prm.sth[pp];
@@ -94,85 +170,77 @@ __global__ void k_diag(const Params prm, const Ptrs P) {
 }
 
 // stokes_drift, umwm_stokes.F90:55-128: util recomputed from k, d and cg0
-// instead of stored (it would be om*im*lm floats).  Per point the
-// direction sums X(o), Y(o) are formed once; the depths are then taken in
-// chunks of SLC with the per-frequency factors computed once per chunk, and
-// the depth-dependent exponentials through ex2 (cosh(x) = (2^(x log2 e) +
-// 2^(-x log2 e)) / 2, which has no cancellation; sinh(kd), which has, stays
-// sinhf).
-__global__ void k_stokes(const Params prm, const Ptrs P) {
-  constexpr int SLC = 8;
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= prm.Ntot) return;
-  const Member& Mb = prm.mem[prm.tile_mem[j / TILE]];
-  if (j >= Mb.ghost) return;
-  const int O = prm.O, NP = prm.P, ldN = prm.ldN, lm = prm.lm;
-  float X[MAX_OM], Y[MAX_OM];
-  for (int o = 0; o < O; ++o) {
-    float x = 0.f, y = 0.f;
-    const float* Eo = P.E + sidx(prm, o, 0, j);
-#pragma unroll 4
-    for (int p = 0; p < NP; ++p) {
-      const float e = Eo[poff(p)];
-      x += e * prm.cth[p];
-      y += e * prm.sth[p];
-    }
-    X[o] = x; Y[o] = y;
-  }
+// instead of stored (it would be om*im*lm floats).  The warps first share out
+// the levels (direction sums times the depth-independent factors, to shared
+// memory: [om][4][32]), then the depths, with the depth-dependent
+// exponentials through ex2 (cosh(x) = (2^(x log2 e) + 2^(-x log2 e)) / 2, which
+// has no cancellation; sinh(kd), which has, stays sinhf); the first warp then
+// finds the e-folding depth from the profile ([lm][32]).
+__global__ void __launch_bounds__(MW * 32) k_stokes(const Params prm, const Ptrs P) {
+  extern __shared__ float sh[];
+  __shared__ float4 cs[MAX_PM / 2];
+  fill_cs(prm, reinterpret_cast<float*>(cs));
+  __syncthreads();
+  const Member& Mb = prm.mem[prm.tile_mem[(blockIdx.x * 32) / TILE]];
+  BlockPoint b;
+  if (!block_point(Mb, b)) return;
+  const int j = b.j, lane = b.lane, w = b.w, O = prm.O, NQ = prm.P / 4, ldN = prm.ldN, lm = prm.lm;
+  float* const um_s = sh + O * 128;
   const float d = P.d[j];
   const float twopi = 2.f * 3.14159274f, log2e = 1.44269504f;
-  float um1 = 0.f, usm_prev = 0.f, ds = 0.f, ust_ef = 0.f;
-  bool found = false;
-  for (int l0 = 0; l0 < lm; l0 += SLC) {
-    float su[SLC], sv[SLC];
-#pragma unroll
-    for (int i = 0; i < SLC; ++i) su[i] = sv[i] = 0.f;
-    for (int o = 0; o < O; ++o) {
-      const float kk = P.TAB[tidx(prm, o, T_K, j)];
-      const float dwn = prm.dom[o] / fabsf(P.TAB[tidx(prm, o, T_CG0, j)]);
-      const float kd = kk * d;
-      const float a = ((twopi * prm.f[o]) * (kk * kk)) * dwn * prm.dth;  // util without its depth factor
-      const float sh = sinhf(kd);
-      const float ish2 = kd > 50.f ? 0.f : 1.f / (sh * sh);
-      const float k2l = 2.f * kk * log2e;
-#pragma unroll
-      for (int i = 0; i < SLC; ++i) {
-        const int l = l0 + i;
-        if (l < lm) {
-          const float dep = prm.depth[l];
-          if (!(fabsf(dep) > d)) {
-            const float arg = 2.f * kk * (dep + d);
-            float u;
-            if (fabsf(arg) > 50.f || kd > 50.f) {
-              u = (2.f * a) * ex2_approx(k2l * dep);
-            } else {
-              const float t = k2l * (dep + d);
-              u = a * (0.5f * (ex2_approx(t) + ex2_approx(-t))) * ish2;
-            }
-            su[i] += u * X[o];
-            sv[i] += u * Y[o];
-          }
-        }
+  for (int o = w; o < O; o += MW) {
+    const float* T = P.TAB + tidx(prm, o, 0, j);
+    const float4* r = reinterpret_cast<const float4*>(P.E + sidx(prm, o, 0, j));
+    float x = 0.f, y = 0.f;
+#pragma unroll 3
+    for (int q = 0; q < NQ; ++q) {
+      const float4 e = r[q * 32], c = cs[2 * q], n = cs[2 * q + 1];
+      x += e.x * c.x + e.y * c.y + e.z * c.z + e.w * c.w;
+      y += e.x * n.x + e.y * n.y + e.z * n.z + e.w * n.w;
+    }
+    const float kk = T[T_K * 32], kd = kk * d;
+    const float a = ((twopi * prm.f[o]) * (kk * kk)) * (prm.dom[o] / fabsf(T[T_CG0 * 32])) * prm.dth;
+    const float s = sinhf(kd);
+    float* q4 = sh + o * 128 + lane;
+    q4[0] = a * x;
+    q4[32] = a * y;
+    q4[64] = 2.f * kk * log2e;
+    q4[96] = kd > 50.f ? -1.f : 1.f / (s * s);  // -1: deep water at every depth
+  }
+  __syncthreads();
+  for (int l = w; l < lm; l += MW) {
+    const float dep = prm.depth[l];
+    float su = 0.f, sv = 0.f;
+    if (!(fabsf(dep) > d)) {
+#pragma unroll 4
+      for (int o = 0; o < O; ++o) {
+        const float* q4 = sh + o * 128 + lane;
+        const float k2l = q4[64], is2 = q4[96], t = k2l * (dep + d);
+        // |2 k (z + d)| > 50 or k d > 50: the deep-water profile
+        const bool deep = is2 < 0.f || fabsf(t) > 50.f * log2e;
+        const float u = deep ? 2.f * ex2_approx(k2l * dep) : (0.5f * (ex2_approx(t) + ex2_approx(-t))) * is2;
+        su = fmaf(u, q4[0], su);
+        sv = fmaf(u, q4[32], sv);
       }
     }
-#pragma unroll
-    for (int i = 0; i < SLC; ++i) {
-      const int l = l0 + i;
-      if (l < lm) {
-        const float dep = prm.depth[l];
-        P.us[(size_t)l * ldN + j] = su[i];
-        P.vs[(size_t)l * ldN + j] = sv[i];
-        const float um = sqrtf(su[i] * su[i] + sv[i] * sv[i]);
-        if (l == 0) {
-          um1 = um;
-          ust_ef = um1 * prm.eulerinv;
-        } else if (um1 != 0.f && !found && um < ust_ef) {
-          ds = (fabsf(usm_prev - ust_ef) * dep + fabsf(um - ust_ef) * prm.depth[l - 1]) / (usm_prev - um);
-          found = true;
-        }
-        usm_prev = um;
-      }
+    if (b.valid) {
+      P.us[(size_t)l * ldN + j] = su;
+      P.vs[(size_t)l * ldN + j] = sv;
     }
+    um_s[l * 32 + lane] = sqrtf(su * su + sv * sv);
+  }
+  __syncthreads();
+  if (w != 0 || !b.valid) return;
+  float ds = 0.f;
+  const float um1 = lm > 0 ? um_s[lane] : 0.f, ust_ef = um1 * prm.eulerinv;
+  float prev = um1;
+  for (int l = 1; l < lm && um1 != 0.f; ++l) {
+    const float um = um_s[l * 32 + lane];
+    if (um < ust_ef) {
+      ds = (fabsf(prev - ust_ef) * prm.depth[l] + fabsf(um - ust_ef) * prm.depth[l - 1]) / (prev - um);
+      break;
+    }
+    prev = um;
   }
   P.ds[j] = -ds;
 }
@@ -262,98 +330,107 @@ __global__ void k_begin_dtg(const Params prm) {
 
 // stress('ocn'), umwm_stress.F90:34-214: per wet point, from the current
 // spectrum and the source terms the last substep of the dtg kept (Sin, Sds
-// after cothkd, Snl, and the ustar of its sdt).  One thread per point; the
-// sums over directions run inside the frequency sums in the reference's
-// order (p outer, o inner per accumulator, then the sum over o with kdk).
-__global__ void k_stress_ocn(const Params prm, const Ptrs P) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= prm.Ntot) return;
-  const Member& M = prm.mem[prm.tile_mem[j / TILE]];
-  if (j >= M.ghost) return;
-  const int ja = apt(M, j);
-  const int O = prm.O, NP = prm.P, oc = P.oc[j];
-  const float rhow = P.rhow[ja], wdir = P.wdir[ja];
-  const float sdtc = (prm.sdt_fac * sqrtf(P.rhorat[ja])) * P.src_ust[j];
-  auto tab = [&](int t, int o) { return P.TAB[tidx(prm, o, t, j)]; };
-  float top_x = 0, top_y = 0, bot_x = 0, bot_y = 0, snl_x = 0, snl_y = 0, eo_x = 0, eo_y = 0, ea_x = 0, ea_y = 0;
-  float tailx = 0, taily = 0;
-  float f1x = 0, f1y = 0, f2x = 0, f2y = 0, f3x = 0, f3y = 0;
-  for (int o = 0; o < O; ++o) {
-    const float cp0 = tab(T_CP0, o), icp = 1.f / cp0, kdk = tab(T_KDK, o), kk = tab(T_K, o);
-    const float sdt = sdtc * kk, sdv = tab(T_SDV, o), sbf = tab(T_SBF, o);
+// after cothkd, Snl, and the ustar of its sdt).  A level's direction sums
+// (e, e Sds, Snl and e Sin times cos th and sin th; e Sin split by the three
+// form-drag classes) are formed first and weighted by the level's factors.
+__global__ void __launch_bounds__(MW * 32) k_stress_ocn(const Params prm, const Ptrs P) {
+  enum { TOPX, TOPY, BOTX, BOTY, SNLX, SNLY, EOX, EOY, EAX, EAY, F1X, F1Y, F2X, F2Y, F3X, F3Y, TX, TY, NS };
+  __shared__ float part[MW][NS][32];
+  __shared__ float4 cs[MAX_PM / 2], cw[MAX_PM / 4 * 32];
+  fill_cs(prm, reinterpret_cast<float*>(cs));
+  const Member& M = prm.mem[prm.tile_mem[(blockIdx.x * 32) / TILE]];
+  BlockPoint b;
+  if (!block_point(M, b)) return;
+  const int j = b.j, lane = b.lane, w = b.w, O = prm.O, NQ = prm.P / 4;
+  const int jj = b.valid ? j : M.ghost, ja = apt(M, jj), oc = b.valid ? P.oc[j] : 0;
+  cw_fill(prm, P.wdir[ja], w, NQ, MW, cw);
+  __syncthreads();
+  const float sdtc = (prm.sdt_fac * sqrtf(P.rhorat[ja])) * P.src_ust[jj];
+  float sum[NS];
+#pragma unroll
+  for (int i = 0; i < NS; ++i) sum[i] = 0.f;
+  for (int o = w; o < O; o += MW) {
+    const float* T = P.TAB + tidx(prm, o, 0, j);
+    const float cp0 = T[T_CP0 * 32], icp = 1.f / cp0, kdk = T[T_KDK * 32], kk = T[T_K * 32];
+    const float sdt = sdtc * kk, sdv = T[T_SDV * 32], sbf = T[T_SBF * 32];
     // downshifting weights at levels o >= 3 (1-based)
     float wm = 0.f, wl = 0.f;
     if (o >= 2) {
-      const float i1 = 1.f / tab(T_CP0, o - 1), i2 = 1.f / tab(T_CP0, o - 2);
+      const float i1 = 1.f / T[(T_CP0 - T_COUNT) * 32], i2 = 1.f / T[(T_CP0 - 2 * T_COUNT) * 32];
       wm = prm.bf1 * cp0 * i1 + prm.bf2 * cp0 * i2;
       wl = prm.bf1 * (1.f - cp0 * i1) + prm.bf2 * (1.f - cp0 * i2);
     }
-    float ux = 0, uy = 0, bx = 0, by = 0, nx = 0, ny = 0, ex = 0, ey = 0, ax = 0, ay = 0;
-    for (int p = 0; p < NP; ++p) {
-      const size_t a = sidx(prm, o, p, j);
-      const float e = P.E[a], sin_ = P.src_sin[a], sds = P.src_sds[a], snl = P.src_snl[a];
-      const float c = prm.cth[p], s = prm.sth[p];
-      ux = ux + e * (sds + sdt + sdv) * c * icp;
-      uy = uy + e * (sds + sdt + sdv) * s * icp;
-      if (o >= 2) {
-        ux = ux - snl * wm * c * icp;
-        uy = uy - snl * wm * s * icp;
-      }
-      bx = bx + e * sbf * c * icp;
-      by = by + e * sbf * s * icp;
-      if (o >= 2 && o < oc) {
-        nx = nx + snl * wl * c * icp;
-        ny = ny + snl * wl * s * icp;
-      }
-      ex = ex + e * sds * c;
-      ey = ey + e * sds * s;
-      if (o >= 2) {
-        ex = ex - snl * wm * c;
-        ey = ey - snl * wm * s;
-      }
-      ax = ax + e * sin_ * c;
-      ay = ay + e * sin_ * s;
-      const float dd = e * sin_ * icp * kdk;
-      if (sin_ > 0.f) {
-        f1x += dd * c; f1y += dd * s;
-      } else if (cosf(wdir - prm.th[p]) < 0.f) {
-        f2x += dd * c; f2y += dd * s;
-      } else {
-        f3x += dd * c; f3y += dd * s;
+    const size_t a0 = sidx(prm, o, 0, j);
+    float ex = 0, ey = 0, dx = 0, dy = 0, nx = 0, ny = 0, g1x = 0, g1y = 0, g2x = 0, g2y = 0, g3x = 0, g3y = 0;
+    for (int q = 0; q < NQ; ++q) {
+      auto row = [&](const float* f) { return *reinterpret_cast<const float4*>(f + a0 + q * 128); };
+      const float4 e4 = row(P.E), i4 = row(P.src_sin), d4 = row(P.src_sds), n4 = row(P.src_snl);
+      const float4 c4 = cs[2 * q], s4 = cs[2 * q + 1], w4 = cw[q * 32 + lane];
+      const float e[4] = {e4.x, e4.y, e4.z, e4.w}, si[4] = {i4.x, i4.y, i4.z, i4.w}, sd[4] = {d4.x, d4.y, d4.z, d4.w};
+      const float sn[4] = {n4.x, n4.y, n4.z, n4.w}, c[4] = {c4.x, c4.y, c4.z, c4.w}, s[4] = {s4.x, s4.y, s4.z, s4.w};
+      const float cwv[4] = {w4.x, w4.y, w4.z, w4.w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float ed = e[i] * sd[i], ei = e[i] * si[i];
+        ex = fmaf(e[i], c[i], ex); ey = fmaf(e[i], s[i], ey);
+        dx = fmaf(ed, c[i], dx); dy = fmaf(ed, s[i], dy);
+        nx = fmaf(sn[i], c[i], nx); ny = fmaf(sn[i], s[i], ny);
+        if (si[i] > 0.f) {
+          g1x = fmaf(ei, c[i], g1x); g1y = fmaf(ei, s[i], g1y);
+        } else if (cwv[i] < 0.f) {
+          g2x = fmaf(ei, c[i], g2x); g2y = fmaf(ei, s[i], g2y);
+        } else {
+          g3x = fmaf(ei, c[i], g3x); g3y = fmaf(ei, s[i], g3y);
+        }
       }
     }
-    top_x += ux * kdk; top_y += uy * kdk;
-    bot_x += bx * kdk; bot_y += by * kdk;
-    snl_x += nx * kdk; snl_y += ny * kdk;
-    eo_x += ex * kdk; eo_y += ey * kdk;
-    ea_x += ax * kdk; ea_y += ay * kdk;
+    const float ux = (dx + ex * (sdt + sdv) - nx * wm) * icp, uy = (dy + ey * (sdt + sdv) - ny * wm) * icp;
+    sum[TOPX] += ux * kdk; sum[TOPY] += uy * kdk;
+    sum[BOTX] += ex * sbf * icp * kdk; sum[BOTY] += ey * sbf * icp * kdk;
+    if (o >= 2 && o < oc) {
+      sum[SNLX] += nx * wl * icp * kdk; sum[SNLY] += ny * wl * icp * kdk;
+    }
+    sum[EOX] += (dx - nx * wm) * kdk; sum[EOY] += (dy - ny * wm) * kdk;
+    sum[EAX] += (g1x + g2x + g3x) * kdk; sum[EAY] += (g1y + g2y + g3y) * kdk;
+    const float ki = icp * kdk;
+    sum[F1X] += g1x * ki; sum[F1Y] += g1y * ki;
+    sum[F2X] += g2x * ki; sum[F2Y] += g2y * ki;
+    sum[F3X] += g3x * ki; sum[F3Y] += g3y * ki;
     if (o == O - 1) {
-      const float tl = stress_tail(P.wspd[ja], kk);
-      tailx = ux * kk * tl * rhow * prm.dthg;
-      taily = uy * kk * tl * rhow * prm.dthg;
+      sum[TX] = ux * kk;
+      sum[TY] = uy * kk;
     }
   }
-  const float rg = rhow * prm.dthg;
+#pragma unroll
+  for (int i = 0; i < NS; ++i) part[w][i][lane] = sum[i];
+  __syncthreads();
+  if (w != 0 || !b.valid) return;
+  for (int v = 1; v < MW; ++v)
+#pragma unroll
+    for (int i = 0; i < NS; ++i) sum[i] += part[v][i][lane];
+  const float rg = P.rhow[ja] * prm.dthg;
+  const float tl = stress_tail(P.wspd[ja], P.TAB[tidx(prm, O - 1, T_K, j)]);
+  const float tailx = sum[TX] * tl * rg, taily = sum[TY] * tl * rg;
   const size_t L = (size_t)prm.ldN;
   float* out = P.ocn;
-  out[OCN_TAUX_TOP * L + j] = top_x * rg + tailx + P.taux_skin[j];
-  out[OCN_TAUY_TOP * L + j] = top_y * rg + taily + P.tauy_skin[j];
-  out[OCN_TAUX_BOT * L + j] = bot_x * rg;
-  out[OCN_TAUY_BOT * L + j] = bot_y * rg;
-  out[OCN_TAUX_SNL * L + j] = snl_x * rg;
-  out[OCN_TAUY_SNL * L + j] = snl_y * rg;
-  out[OCN_EPSX_OCN * L + j] = eo_x * rg;
-  out[OCN_EPSY_OCN * L + j] = eo_y * rg;
-  out[OCN_EPSX_ATM * L + j] = ea_x * rg;
-  out[OCN_EPSY_ATM * L + j] = ea_y * rg;
+  out[OCN_TAUX_TOP * L + j] = sum[TOPX] * rg + tailx + P.taux_skin[j];
+  out[OCN_TAUY_TOP * L + j] = sum[TOPY] * rg + taily + P.tauy_skin[j];
+  out[OCN_TAUX_BOT * L + j] = sum[BOTX] * rg;
+  out[OCN_TAUY_BOT * L + j] = sum[BOTY] * rg;
+  out[OCN_TAUX_SNL * L + j] = sum[SNLX] * rg;
+  out[OCN_TAUY_SNL * L + j] = sum[SNLY] * rg;
+  out[OCN_EPSX_OCN * L + j] = sum[EOX] * rg;
+  out[OCN_EPSY_OCN * L + j] = sum[EOY] * rg;
+  out[OCN_EPSX_ATM * L + j] = sum[EAX] * rg;
+  out[OCN_EPSY_ATM * L + j] = sum[EAY] * rg;
   out[OCN_TAILX * L + j] = tailx;
   out[OCN_TAILY * L + j] = taily;
-  out[OCN_TAUX1 * L + j] = f1x * rg;
-  out[OCN_TAUY1 * L + j] = f1y * rg;
-  out[OCN_TAUX2 * L + j] = f2x * rg;
-  out[OCN_TAUY2 * L + j] = f2y * rg;
-  out[OCN_TAUX3 * L + j] = f3x * rg;
-  out[OCN_TAUY3 * L + j] = f3y * rg;
+  out[OCN_TAUX1 * L + j] = sum[F1X] * rg;
+  out[OCN_TAUY1 * L + j] = sum[F1Y] * rg;
+  out[OCN_TAUX2 * L + j] = sum[F2X] * rg;
+  out[OCN_TAUY2 * L + j] = sum[F2Y] * rg;
+  out[OCN_TAUX3 * L + j] = sum[F3X] * rg;
+  out[OCN_TAUY3 * L + j] = sum[F3Y] * rg;
 }
 
 // Graph-driven inner loop: arm before the graph launch, then after each
@@ -399,15 +476,16 @@ cudaError_t launch_dts(const Params& prm, const Ptrs& P, int compute_rot, int fi
   return cudaGetLastError();
 }
 cudaError_t launch_sice(const Params& prm, const Ptrs& P, cudaStream_t st) {
-  k_sice<<<(prm.Ntot + 127) / 128, 128, 0, st>>>(prm, P);
+  k_sice<<<prm.Ntot / 32, MW * 32, 0, st>>>(prm, P);
   return cudaGetLastError();
 }
 cudaError_t launch_diag(const Params& prm, const Ptrs& P, cudaStream_t st) {
-  k_diag<<<(prm.Ntot + 127) / 128, 128, 0, st>>>(prm, P);
+  k_diag<<<prm.Ntot / 32, MW * 32, 0, st>>>(prm, P);
   return cudaGetLastError();
 }
 cudaError_t launch_stokes(const Params& prm, const Ptrs& P, cudaStream_t st) {
-  k_stokes<<<(prm.Ntot + 127) / 128, 128, 0, st>>>(prm, P);
+  // at most 64 levels x 512 + 100 depths x 128 bytes
+  k_stokes<<<prm.Ntot / 32, MW * 32, (size_t)(prm.O * 128 + prm.lm * 32) * sizeof(float), st>>>(prm, P);
   return cudaGetLastError();
 }
 cudaError_t launch_screen(const Params& prm, const Ptrs& P, cudaStream_t st) {
@@ -436,7 +514,7 @@ cudaError_t launch_begin_dtg(const Params& prm, cudaStream_t st) {
   return cudaGetLastError();
 }
 cudaError_t launch_stress_ocn(const Params& prm, const Ptrs& P, cudaStream_t st) {
-  k_stress_ocn<<<(prm.Ntot + 127) / 128, 128, 0, st>>>(prm, P);
+  k_stress_ocn<<<prm.Ntot / 32, MW * 32, 0, st>>>(prm, P);
   return cudaGetLastError();
 }
 cudaError_t launch_loop_arm(Global* g, int budget, cudaStream_t st) {

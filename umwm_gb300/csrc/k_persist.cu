@@ -123,7 +123,7 @@ __global__ void __launch_bounds__(128, UMWM_PERSIST_MINB)
     forcing_stage(prm, P, nb, compute_rot);
     if (!bar_s(0)) return;
     if (prm.ice_possible) {
-      for (int j = blockIdx.x * 128 + threadIdx.x; j < prm.Ntot; j += nb * 128) sice_point(prm, P, j);
+      for (int j = blockIdx.x * 128 + threadIdx.x; j < prm.Ntot; j += nb * 128) sice_point(prm, P, j, 8);
       if (!bar_s(1)) return;
     }
     for (int v = blockIdx.x; v < nvb; v += nb) {

@@ -204,20 +204,38 @@ __device__ __forceinline__ void dts_body(const Params& prm, const Ptrs& P, int c
   if (threadIdx.x == 0) P.glob->not_done = left;
 }
 
-// s_ice for wet point j: significant wave height where fice > fice_lth and
-// the attenuation factor (umwm_source_functions.F90:108-153).
-__device__ __forceinline__ void sice_point(const Params& prm, const Ptrs& P, int j) {
+// s_ice (umwm_source_functions.F90:108-153): the energy sum of the levels
+// o0, o0 + step, ... of point j, and the attenuation factor of the whole sum
+// (C1 Hs, Hs at most 3 m).
+__device__ __forceinline__ float sice_levels(const Params& prm, const Ptrs& P, int j, int o0, int step) {
+  float h = 0.f;
+  for (int o = o0; o < prm.O; o += step) {
+    const float4* r = reinterpret_cast<const float4*>(P.E + sidx(prm, o, 0, j));
+    float s = 0.f;
+#pragma unroll 3
+    for (int q = 0; q < prm.P / 4; ++q) {
+      const float4 e = r[q * 32];
+      s += (e.x + e.y) + (e.z + e.w);
+    }
+    h = fmaf(s, P.TAB[tidx(prm, o, T_KDK, j)], h);
+  }
+  return h;
+}
+__device__ __forceinline__ float sice_factor(const Params& prm, float h) {
+  h = 4.f * sqrtf(h * prm.dth);
+  const float C1 = -5.35e-6f;
+  return (h < 3.f) ? C1 * h : C1 * 3.f;
+}
+// the same by one thread, its sum in the parts of `parts` warps (the
+// persistent kernel: the same bits as k_sice)
+__device__ __forceinline__ void sice_point(const Params& prm, const Ptrs& P, int j, int parts) {
   const Member& M = prm.mem[prm.tile_mem[j / TILE]];
   if (j >= M.ghost || M.ctl->done) return;
   float sv = 0.f;
   if (P.fice[apt(M, j)] > prm.fice_lth) {
     float h = 0.f;
-    for (int p = 0; p < prm.P; ++p)
-      for (int o = 0; o < prm.O; ++o)
-        h += P.E[sidx(prm, o, p, j)] * P.TAB[tidx(prm, o, T_KDK, j)];
-    h = 4.f * sqrtf(h * prm.dth);
-    const float C1 = -5.35e-6f;
-    sv = (h < 3.f) ? C1 * h : C1 * 3.f;
+    for (int i = 0; i < parts; ++i) h += sice_levels(prm, P, j, i, parts);
+    sv = sice_factor(prm, h);
   }
   P.sice_v[j] = sv;
 }
