@@ -155,6 +155,7 @@ struct Global {
   int iters;               // substeps the graph-driven inner loop ran since it was armed
   int nonfinite;           // non-finite values found by the last finite check
   int save_src;            // the last substep of this dtg keeps its source terms (for stress('ocn'))
+  unsigned phys_blocks;    // blocks of the dts pre-pass that are through (back at 0 after it)
   unsigned long long cut_count;  // bins whose negative ef the propagation cut to 0 (option "count_cut")
   // grid barrier of the persistent substep kernel: arrivals, generation,
   // and the error flag a timed-out wait sets (reset before each launch)

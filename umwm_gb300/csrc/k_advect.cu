@@ -36,6 +36,7 @@
 // of warps) and finishes the drag, skin stress and ustar.
 #include "kernels.hpp"
 #include "adv_body.cuh"
+#include "misc_body.cuh"
 
 namespace umwm {
 
@@ -47,6 +48,14 @@ __global__ void __launch_bounds__(W * 32, MINB) k_advect(const Params prm, const
   __shared__ float4 dirs[NP / 4 * DIR_ROWS], cw[NP / 4 * 32];
   dir_fill<NP>(prm, reinterpret_cast<float*>(dirs));  // (advect_body's barrier)
   advect_body<NP, CURV, CNT, false>(prm, P, blockIdx.x, adv_smem_u32(dirs), cw, dsm, dsm + adv_red_floats(prm.O));
+  // the block of a member's print point (its first block without one) writes
+  // the member's screen line and counts the substep; a kernel of its own took
+  // 8 to 14 us a substep, this 0 to 2 us
+  const Member& M = prm.mem[prm.tile_mem[(blockIdx.x * 32) / TILE]];
+  if ((M.iip >= 0 ? M.iip : M.off) >> 5 == blockIdx.x) {
+    __syncthreads();  // this block's spectrum and stress are written
+    screen_member<256>(prm, P, M, dsm, dsm + 256);
+  }
 }
 
 template <int NP, bool CURV, int W, int MINB, bool CNT = false>

@@ -1,6 +1,6 @@
-// Per-substep forcing and cut-off kernel, the dts/dtr control kernel, and the
-// once-per-output kernels: diag, Stokes drift, sea-ice Hs, the screen line
-// and the spectrum layout transposes.
+// Per-substep forcing and cut-off kernel, the sea-ice Hs, and the
+// once-per-output kernels: diag, Stokes drift, stress('ocn') and the spectrum
+// layout transposes.
 #include <algorithm>
 #include <cfloat>
 
@@ -20,13 +20,6 @@ __global__ void k_prep(const Params prm, const Ptrs P, int compute_rot) {
   if (ctl->done) return;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < M.NM; i += gridDim.x * blockDim.x)
     prep_point(prm, P, M, ctl, i, compute_rot);
-}
-
-// source(): dts = min(min_i physics_time_step, dtamin, dtg - sumt), the
-// first-step rule and sumt update (umwm_physics.F90:41-58); refraction's
-// dtr (umwm_advection.F90:145-158).  One thread.
-__global__ void k_dts(const Params prm, const Ptrs P, int compute_rot, int first) {
-  dts_body(prm, P, compute_rot, first);
 }
 
 // The once-per-interval kernels below and the sea-ice wave height share one
@@ -245,13 +238,6 @@ __global__ void __launch_bounds__(MW * 32) k_stokes(const Params prm, const Ptrs
   P.ds[j] = -ds;
 }
 
-// Screen line at the print point (umwm_top.F90:143-148, umwm_util.F90:69-124);
-// also clears 'first' after the first substep.
-__global__ void k_screen(const Params prm, const Ptrs P) {
-  __shared__ float s0[256], s2[256];
-  screen_member<256, 256>(prm, P, blockIdx.x, s0, s2);
-}
-
 // Reference order F(om,pm,im) (o fastest) <-> the blocked device layout, one
 // CTA per 32 wet points (from `off`, which need not start a block) and four
 // directions: reads of 16 bytes per point and level, rows of 4 om floats per
@@ -433,18 +419,11 @@ __global__ void __launch_bounds__(MW * 32) k_stress_ocn(const Params prm, const 
   out[OCN_TAUY3 * L + j] = sum[F3Y] * rg;
 }
 
-// Graph-driven inner loop: arm before the graph launch, then after each
-// substep count it and set the while node's condition (another substep while
-// a member is inside the dtg and the budget lasts).
+// Graph-driven inner loop: arm before the graph launch; each substep's dts
+// counts it and sets the while node's condition.
 __global__ void k_loop_arm(Global* g, int budget) {
   g->budget = budget;
   g->iters = 0;
-}
-
-__global__ void k_loop_cond(Global* g, cudaGraphConditionalHandle h) {
-  g->iters += 1;
-  if (g->budget > 0) g->budget -= 1;
-  cudaGraphSetConditional(h, (g->not_done && g->budget != 0) ? 1u : 0u);
 }
 
 // Count the NaN/Inf values of a[0..n) into *count (option "check_finite").
@@ -471,10 +450,6 @@ cudaError_t launch_prep(const Params& prm, const Ptrs& P, int compute_rot, int m
   k_prep<<<grid, 256, 0, st>>>(prm, P, compute_rot);
   return cudaGetLastError();
 }
-cudaError_t launch_dts(const Params& prm, const Ptrs& P, int compute_rot, int first, cudaStream_t st) {
-  k_dts<<<1, 256, 0, st>>>(prm, P, compute_rot, first);
-  return cudaGetLastError();
-}
 cudaError_t launch_sice(const Params& prm, const Ptrs& P, cudaStream_t st) {
   k_sice<<<prm.Ntot / 32, MW * 32, 0, st>>>(prm, P);
   return cudaGetLastError();
@@ -486,10 +461,6 @@ cudaError_t launch_diag(const Params& prm, const Ptrs& P, cudaStream_t st) {
 cudaError_t launch_stokes(const Params& prm, const Ptrs& P, cudaStream_t st) {
   // at most 64 levels x 512 + 100 depths x 128 bytes
   k_stokes<<<prm.Ntot / 32, MW * 32, (size_t)(prm.O * 128 + prm.lm * 32) * sizeof(float), st>>>(prm, P);
-  return cudaGetLastError();
-}
-cudaError_t launch_screen(const Params& prm, const Ptrs& P, cudaStream_t st) {
-  k_screen<<<prm.nmem, 256, 0, st>>>(prm, P);
   return cudaGetLastError();
 }
 template <bool TO_REF>
@@ -519,10 +490,6 @@ cudaError_t launch_stress_ocn(const Params& prm, const Ptrs& P, cudaStream_t st)
 }
 cudaError_t launch_loop_arm(Global* g, int budget, cudaStream_t st) {
   k_loop_arm<<<1, 1, 0, st>>>(g, budget);
-  return cudaGetLastError();
-}
-cudaError_t launch_loop_cond(Global* g, cudaGraphConditionalHandle h, cudaStream_t st) {
-  k_loop_cond<<<1, 1, 0, st>>>(g, h);
   return cudaGetLastError();
 }
 cudaError_t launch_count_nonfinite(const float* a, size_t n, int* count, cudaStream_t st) {

@@ -140,7 +140,10 @@ __global__ void __launch_bounds__(128, UMWM_PERSIST_MINB)
       __syncthreads();  // the next block reuses the sums
     }
     if (!bar_s(5)) return;
-    for (int m = blockIdx.x; m < prm.nmem; m += nb) screen_member<256, 128>(prm, P, m, scr[0], scr[1]);
+    for (int m = blockIdx.x; m < prm.nmem; m += nb) {
+      screen_member<256>(prm, P, prm.mem[m], scr[0], scr[1]);
+      __syncthreads();  // the next member reuses the sums
+    }
     if (blockIdx.x == 0 && threadIdx.x == 0) gl->iters += 1;
     if (!bar_s(6)) return;
     // not_done was set by this substep's dts, two barriers ago

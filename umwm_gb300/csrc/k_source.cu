@@ -38,30 +38,61 @@
 #include <algorithm>
 
 #include "kernels.hpp"
+#include "misc_body.cuh"
 #include "src_body.cuh"
 
 namespace umwm {
 
-template <int NP, int W, int MINB, int TMA = 0>
-__global__ void __launch_bounds__(W * 32, MINB) k_phys(const Params prm, const Ptrs P, int compute_rot) {
+// dts of the substep, and in a graph its count and the while node's condition
+__device__ __forceinline__ void dts_end(const Params& prm, const Ptrs& P, int compute_rot, const SubstepEnd& end) {
+  const int left = dts_body(prm, P, compute_rot, end.first);
+  if (threadIdx.x == 0 && end.in_graph) {
+    Global* g = P.glob;
+    g->iters += 1;
+    if (g->budget > 0) g->budget -= 1;
+    cudaGraphSetConditional(end.loop, (left && g->budget != 0) ? 1u : 0u);
+  }
+}
+
+// END: the last block through forms dts (dts_fused); compiled in only where it
+// is used, since its registers cost the other form 3% at 305 k points.
+template <int NP, int W, int MINB, int TMA, bool END>
+__global__ void __launch_bounds__(W * 32, MINB)
+    k_phys(const Params prm, const Ptrs P, int compute_rot, const SubstepEnd end) {
+  __shared__ int last;
   extern __shared__ __align__(128) float dsm[];
   __shared__ float red[W * 64];
   __shared__ float4 dirs[NP / 4 * DIR_ROWS], cw[NP / 4 * 32];
   __shared__ __align__(8) unsigned long long mbar[TMA ? 2 * W : 1];
   dir_fill<NP>(prm, reinterpret_cast<float*>(dirs));  // (phys_body's barrier)
   phys_body<NP, TMA>(prm, P, compute_rot, blockIdx.x, adv_smem_u32(dirs), cw, red, dsm, adv_smem_u32(mbar));
+  if constexpr (!END) return;
+  // thread 0 of each block wrote the block's minimum and maximum
+  if (threadIdx.x == 0) {
+    __threadfence();
+    last = atomicAdd(&P.glob->phys_blocks, 1u) == gridDim.x - 1;
+    __threadfence();
+  }
+  __syncthreads();
+  if (!last) return;
+  if (threadIdx.x == 0) P.glob->phys_blocks = 0;
+  dts_end(prm, P, compute_rot, end);
+}
+__global__ void k_dts(const Params prm, const Ptrs P, int compute_rot, const SubstepEnd end) {
+  dts_end(prm, P, compute_rot, end);
 }
 
-template <int NP, int W, int MINB, int TMA = 0>
-static cudaError_t go_phys(const Params& prm, const Ptrs& P, int compute_rot, int warps, cudaStream_t st) {
+template <int NP, int W, int MINB, int TMA = 0, bool END = (W == 16)>
+static cudaError_t go_phys(const Params& prm, const Ptrs& P, int compute_rot, const SubstepEnd& end, int warps,
+                           cudaStream_t st) {
   const size_t smem = TMA ? (size_t)warps * 2 * NP * 32 * sizeof(float) : 0;
   if (TMA) {
     static std::atomic<unsigned long long> done{0};
     const cudaError_t e =
-        allow_smem((const void*)k_phys<NP, W, MINB, TMA>, (size_t)W * 2 * NP * 32 * sizeof(float), done);
+        allow_smem((const void*)k_phys<NP, W, MINB, TMA, END>, (size_t)W * 2 * NP * 32 * sizeof(float), done);
     if (e != cudaSuccess) return e;
   }
-  k_phys<NP, W, MINB, TMA><<<prm.Ntot / 32, warps * 32, smem, st>>>(prm, P, compute_rot);
+  k_phys<NP, W, MINB, TMA, END><<<prm.Ntot / 32, warps * 32, smem, st>>>(prm, P, compute_rot, end);
   return cudaGetLastError();
 }
 
@@ -70,14 +101,16 @@ static cudaError_t go_phys(const Params& prm, const Ptrs& P, int compute_rot, in
 // form that loads its rows itself, with prm.minb_phys the resident CTAs its
 // register budget is sized for.
 template <int NP>
-static cudaError_t launch_phys_np(const Params& prm, const Ptrs& P, int compute_rot, cudaStream_t st) {
-  if (prm.groups4_phys) return go_phys<NP, 16, 1>(prm, P, compute_rot, prm.Ntot / 32 <= prm.nsm ? 16 : 8, st);
+static cudaError_t launch_phys_np(const Params& prm, const Ptrs& P, int compute_rot, const SubstepEnd& end,
+                                  cudaStream_t st) {
+  if (prm.groups4_phys) return go_phys<NP, 16, 1>(prm, P, compute_rot, end, prm.Ntot / 32 <= prm.nsm ? 16 : 8, st);
   if constexpr (NP == 36) {
-    if (prm.phys_tma) return go_phys<NP, 4, 5, 1>(prm, P, compute_rot, 4, st);
-    if (prm.minb_phys == 5) return go_phys<NP, 4, 5>(prm, P, compute_rot, 4, st);
-    if (prm.minb_phys == 7) return go_phys<NP, 4, 7>(prm, P, compute_rot, 4, st);
+    if (prm.phys_tma && end.fused) return go_phys<NP, 4, 5, 1, true>(prm, P, compute_rot, end, 4, st);
+    if (prm.phys_tma) return go_phys<NP, 4, 5, 1>(prm, P, compute_rot, end, 4, st);
+    if (prm.minb_phys == 5) return go_phys<NP, 4, 5>(prm, P, compute_rot, end, 4, st);
+    if (prm.minb_phys == 7) return go_phys<NP, 4, 7>(prm, P, compute_rot, end, 4, st);
   }
-  return go_phys<NP, 4, 6>(prm, P, compute_rot, 4, st);
+  return go_phys<NP, 4, 6>(prm, P, compute_rot, end, 4, st);
 }
 
 // The integration: NG direction groups x nc level chunks of one block per CTA.
@@ -128,8 +161,13 @@ static cudaError_t launch_integ_np(const Params& prm, const Ptrs& P, cudaStream_
     default: return cudaErrorInvalidConfiguration; \
   }
 
-cudaError_t launch_source_phys(const Params& prm, const Ptrs& P, int compute_rot, cudaStream_t st) {
-  UMWM_ALL_NP(launch_phys_np, prm, P, compute_rot, st)
+cudaError_t launch_source_phys(const Params& prm, const Ptrs& P, int compute_rot, const SubstepEnd& end,
+                               cudaStream_t st) {
+  UMWM_ALL_NP(launch_phys_np, prm, P, compute_rot, end, st)
+}
+cudaError_t launch_dts(const Params& prm, const Ptrs& P, int compute_rot, const SubstepEnd& end, cudaStream_t st) {
+  k_dts<<<1, 128, 0, st>>>(prm, P, compute_rot, end);
+  return cudaGetLastError();
 }
 cudaError_t launch_source_integ(const Params& prm, const Ptrs& P, cudaStream_t st) {
   UMWM_ALL_NP(launch_integ_np, prm, P, st)

@@ -170,8 +170,10 @@ __device__ __forceinline__ void prep_points(const Params& prm, const Ptrs& P, co
 
 // source(): dts = min(min_i physics_time_step, dtamin, dtg - sumt), the
 // first-step rule and sumt update (umwm_physics.F90:41-58); refraction's
-// dtr (umwm_advection.F90:145-158).  One block, members over its threads.
-__device__ __forceinline__ void dts_body(const Params& prm, const Ptrs& P, int compute_rot, int first) {
+// dtr (umwm_advection.F90:145-158).  One block, members over its threads; the
+// pre-pass's minima and maxima may come from other blocks of the same kernel,
+// so they are read from L2.  Returns whether a member is still inside its dtg.
+__device__ __forceinline__ int dts_body(const Params& prm, const Ptrs& P, int compute_rot, int first) {
   int left = 0;
   for (int m = threadIdx.x; m < prm.nmem; m += blockDim.x) {
     const Member& M = prm.mem[m];
@@ -180,14 +182,14 @@ __device__ __forceinline__ void dts_body(const Params& prm, const Ptrs& P, int c
       c.running = 0;
       continue;
     }
-    float mn = dec_ord_d(c.minphys_enc);
+    float mn = dec_ord_d(__ldcg(&c.minphys_enc));
     float dts = fminf(fminf(mn, M.dtamin), prm.dtg - c.sumt);
     if (!prm.restart && first) dts = 0.f;
     c.dts = dts;
     c.dta = dts;
     c.sumt = c.sumt + dts;
     if (compute_rot) {
-      float mx = dec_ord_d(c.maxrot_enc);
+      float mx = dec_ord_d(__ldcg(&c.maxrot_enc));
       c.dtr_temp = (mx <= FLT_MIN) ? dts : prm.dth / mx;
     }
     c.dtr = fminf(c.dtr_temp, dts);
@@ -202,6 +204,7 @@ __device__ __forceinline__ void dts_body(const Params& prm, const Ptrs& P, int c
   }
   left = __syncthreads_count(left > 0) ? 1 : 0;  // any member left in this block
   if (threadIdx.x == 0) P.glob->not_done = left;
+  return left;
 }
 
 // s_ice (umwm_source_functions.F90:108-153): the energy sum of the levels
@@ -243,19 +246,28 @@ __device__ __forceinline__ void sice_point(const Params& prm, const Ptrs& P, int
 // Screen line of member m at its print point (umwm_top.F90:143-148,
 // umwm_util.F90:69-124); also clears 'first' and counts the substep.  The
 // sums run over V virtual threads (bins strided by V, then a tree
-// reduction), carried by the NT <= V threads of the block, so that any NT
-// gives the same result bit for bit.
-template <int V, int NT>
-__device__ __forceinline__ void screen_member(const Params& prm, const Ptrs& P, int m, float (&s0)[V],
-                                              float (&s2)[V]) {
-  static_assert(V % NT == 0, "virtual threads must be a multiple of the block");
-  const Member& M = prm.mem[m];
+// reduction), carried by the threads of the block, so that any number of them
+// gives the same result bit for bit.  s0, s2: V floats of shared memory each.
+template <int V>
+__device__ __forceinline__ void screen_member(const Params& prm, const Ptrs& P, const Member& M, float* s0, float* s2) {
+  const int NT = blockDim.x;
   Ctl& c = *M.ctl;
   if (!c.running) return;
   const int j = M.iip;
+  double line[6];
+  if (threadIdx.x == 0 && j >= 0) {
+    const int ja = apt(M, j);
+    line[0] = c.sumt / prm.dtg;
+    line[1] = c.dts;
+    line[2] = P.wspd[ja];
+    line[3] = P.wdir[ja];
+    line[4] = P.cd[j] * 1e3f;
+    line[5] = prm.f[P.oc[j] - 1];
+  }
   for (int v = threadIdx.x; v < V; v += NT) {
     float a = 0.f, b = 0.f;
     if (j >= 0) {
+#pragma unroll 6
       for (int b_ = v; b_ < prm.O * prm.P; b_ += V) {
         const int o = b_ / prm.P, p = b_ % prm.P;
         const float ek = P.E[sidx(prm, o, p, j)] * P.TAB[tidx(prm, o, T_KDK, j)];
@@ -267,23 +279,28 @@ __device__ __forceinline__ void screen_member(const Params& prm, const Ptrs& P, 
     s2[v] = b;
   }
   __syncthreads();
-  for (int s = V / 2; s > 0; s >>= 1) {
+  for (int s = V / 2; s >= 32; s >>= 1) {
     for (int v = threadIdx.x; v < s; v += NT) { s0[v] += s0[v + s]; s2[v] += s2[v + s]; }
     __syncthreads();
+  }
+  if (threadIdx.x >= 32) return;
+  float a = s0[threadIdx.x], b = s2[threadIdx.x];
+  for (int s = 16; s > 0; s >>= 1) {
+    a += __shfl_down_sync(0xffffffffu, a, s);
+    b += __shfl_down_sync(0xffffffffu, b, s);
   }
   if (threadIdx.x == 0) {
     const int r = c.log_count;
     if (r < M.log_cap && j >= 0) {
       double* L = M.log + (size_t)r * 8;
-      const int ja = apt(M, j);
-      L[0] = c.sumt / prm.dtg;
-      L[1] = c.dts;
-      L[2] = P.wspd[ja];
-      L[3] = P.wdir[ja];
-      L[4] = 4.f * sqrtf(s0[0] * prm.dth);
-      L[5] = sqrtf(s0[0] / s2[0]);
-      L[6] = P.cd[j] * 1e3f;
-      L[7] = prm.f[P.oc[j] - 1];
+      L[0] = line[0];
+      L[1] = line[1];
+      L[2] = line[2];
+      L[3] = line[3];
+      L[4] = 4.f * sqrtf(a * prm.dth);
+      L[5] = sqrtf(a / b);
+      L[6] = line[4];
+      L[7] = line[5];
       c.log_count = r + 1;
     }
     c.substep += 1;

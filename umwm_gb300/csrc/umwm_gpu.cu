@@ -1366,15 +1366,17 @@ int ensure_ocn(Model& M) {
   return UMWM_OK;
 }
 
-// Enqueue the launches of one substep: prep, [sice], phys, dts, integ,
-// advect, [diag on the first substep of a run], screen.
-int enqueue_substep(Model& M, int compute_rot, int first, bool diag) {
+// Enqueue the launches of one substep: prep, [sice], phys, [dts], integ,
+// advect (with the screen line), [diag on the first substep of a run].  `loop`:
+// the while node of the graph that is being captured.
+int enqueue_substep(Model& M, int compute_rot, int first, bool diag, const cudaGraphConditionalHandle* loop = nullptr) {
   const Params& prm = M.prm;
   const Ptrs& P = M.P;
+  const SubstepEnd end{first, dts_fused(prm) ? 1 : 0, loop ? 1 : 0, loop ? *loop : 0};
   CU(timed(M, K_PREP, [&] { return launch_prep(prm, P, compute_rot, M.max_nm, M.st); }));
   if (prm.ice_possible) CU(timed(M, K_SICE, [&] { return launch_sice(prm, P, M.st); }));
-  CU(tuned(M, TK_PHYS, K_PHYS, [&] { return launch_source_phys(prm, P, compute_rot, M.st); }));
-  CU(timed(M, K_DTS, [&] { return launch_dts(prm, P, compute_rot, first, M.st); }));
+  CU(tuned(M, TK_PHYS, K_PHYS, [&] { return launch_source_phys(prm, P, compute_rot, end, M.st); }));
+  if (!end.fused) CU(timed(M, K_DTS, [&] { return launch_dts(prm, P, compute_rot, end, M.st); }));
   int rc;
   if (sur::active()) {
     // learned source step; points outside its energy budget fall back to
@@ -1389,11 +1391,12 @@ int enqueue_substep(Model& M, int compute_rot, int first, bool diag) {
   }
   CU(tuned(M, TK_ADVECT, K_ADVECT, [&] { return launch_advect(prm, P, M.st); }));
   if (diag) CU(timed(M, K_DIAG, [&] { return launch_diag(prm, P, M.st); }));
-  CU(timed(M, K_SCREEN, [&] { return launch_screen(prm, P, M.st); }));
   return UMWM_OK;
 }
 
-int substep_launches(const Model& M, bool diag) { return 6 + (M.prm.ice_possible ? 1 : 0) + (diag ? 1 : 0); }
+int substep_launches(const Model& M, bool diag) {
+  return 4 + (dts_fused(M.prm) ? 0 : 1) + (M.prm.ice_possible ? 1 : 0) + (diag ? 1 : 0);
+}
 
 int substep(Model& M) {
   const bool first = M.first;
@@ -1419,9 +1422,9 @@ int substep(Model& M) {
 }
 
 // The inner loop of umwm_run as a CUDA graph: one while node whose body is a
-// substep (after the first of a run: compute_rot = currents, first = 0)
-// followed by k_loop_cond, which keeps the loop going while a member is
-// inside the dtg and the armed budget lasts.  Launch parameters are fixed
+// substep (after the first of a run: compute_rot = currents, first = 0); its
+// dts keeps the loop going while a member is inside the dtg and the armed
+// budget lasts.  Launch parameters are fixed
 // after initialize (forcing updates are device copies into fixed buffers), so
 // the graph is built once per model.
 int build_graph(Model& M) {
@@ -1440,13 +1443,11 @@ int build_graph(Model& M) {
   CU(cudaStreamBeginCaptureToGraph(M.st, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
   const bool kt = M.ktime;
   M.ktime = false;
-  int rc = enqueue_substep(M, M.prm.currents ? 1 : 0, 0, false);
-  cudaError_t e = rc ? cudaSuccess : launch_loop_cond(M.d_glob, h, M.st);
+  int rc = enqueue_substep(M, M.prm.currents ? 1 : 0, 0, false, &h);
   M.ktime = kt;
   cudaGraph_t captured = nullptr;
   cudaError_t ec = cudaStreamEndCapture(M.st, &captured);
   if (rc) return rc;
-  CU(e);
   CU(ec);
   CU(cudaGraphInstantiate(&M.graph_exec, M.graph, 0));
   return UMWM_OK;
@@ -1576,7 +1577,7 @@ int run_impl(Model& M, const std::string& start, const std::string& stop) {
         CU(cudaStreamSynchronize(M.st));
         const int it = M.flag_h->iters;
         M.substeps += it;
-        M.launches += 1 + (long long)it * (substep_launches(M, false) + 1);
+        M.launches += 1 + (long long)it * substep_launches(M, false);
         inner += it;
         if (M.flag_h->not_done == 0) break;
         continue;
