@@ -18,8 +18,10 @@ __global__ void k_prep(const Params prm, const Ptrs P, int compute_rot) {
   const Member& M = prm.mem[blockIdx.y];
   Ctl* ctl = M.ctl;
   if (ctl->done) return;
+  bool cur = false;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < M.NM; i += gridDim.x * blockDim.x)
-    prep_point(prm, P, M, ctl, i, compute_rot);
+    cur |= prep_points<1>(prm, P, M, ctl, i, 0, compute_rot);
+  set_anycurrent(ctl, cur);
 }
 
 // The once-per-interval kernels below and the sea-ice wave height share one

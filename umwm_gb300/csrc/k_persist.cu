@@ -76,8 +76,10 @@ __device__ __forceinline__ void forcing_stage(const Params& prm, const Ptrs& P, 
     const Member& M = prm.mem[m];
     Ctl* ctl = M.ctl;
     if (ctl->done) continue;
+    bool cur = false;
     for (int i = blockIdx.x * 128 + threadIdx.x; i < M.NM; i += U * nb * 128)
-      prep_points<U>(prm, P, M, ctl, i, nb * 128, compute_rot);
+      cur |= prep_points<U>(prm, P, M, ctl, i, nb * 128, compute_rot);
+    set_anycurrent(ctl, cur);
   }
 }
 

@@ -21,63 +21,17 @@ __device__ __forceinline__ int cutoff_level(const Params& prm, float fc) {
   return a >= 0 ? a + 1 : 1;
 }
 
-// ctl->anycurrent = 1 where cur holds, one store per warp (every lane of
-// the warp's active set calls this)
+// ctl->anycurrent = 1 where cur holds for a thread of the block (every thread
+// calls this once, after its points): one store per block, none once it is set
 __device__ __forceinline__ void set_anycurrent(Ctl* ctl, bool cur) {
-  const unsigned act = __activemask();
-  if (__any_sync(act, cur) && (threadIdx.x & 31) == __ffs(act) - 1) ctl->anycurrent = 1;
+  if (__syncthreads_or(cur) && threadIdx.x == 0 && __ldcg(&ctl->anycurrent) == 0) ctl->anycurrent = 1;
 }
 
 // One all-point index i of member M (its forcing interpolation at sumt; for
-// wet points also oc, oc_rot and the sheltering coefficient): the per-stage
-// kernel's form, one point per thread (0.13 ms at 1000x1000, against 0.27
-// measured for prep_points<1>, which takes 40 registers instead of 30).
-// prep_points below computes the same values by the same expressions.
-__device__ __forceinline__ void prep_point(const Params& prm, const Ptrs& P, const Member& M, Ctl* ctl, int i,
-                                           int compute_rot) {
-  const float sumt = ctl->sumt, dtg = prm.dtg;
-  const float a = 1.f - sumt / dtg;
-  const int q = (M.mi[i] - 1) + (M.ni[i] - 1) * M.mm;
-  const int ia = M.nmoff + i;
-  if (prm.winds) {
-    float uw = M.uwb[q] * a + M.uwf[q] * sumt / dtg;
-    float vw = M.vwb[q] * a + M.vwf[q] * sumt / dtg;
-    if (prm.gustiness > 0.f) {  // umwm_forcing.F90:49-61
-      const float gu = prm.gustiness * (2.f * gust_uniform(prm.gust_seed, ctl->substep, q, 0) - 1.f);
-      const float gv = prm.gustiness * (2.f * gust_uniform(prm.gust_seed, ctl->substep, q, 1) - 1.f);
-      uw = uw * (1.f + gu);
-      vw = vw * (1.f + gv);
-    }
-    P.wspd[ia] = sqrtf(uw * uw + vw * vw);
-    P.wdir[ia] = atan2f(vw, uw);
-  }
-  if (prm.seaice) P.fice[ia] = M.ficeb[q] * a + M.ficef[q] * sumt / dtg;
-  if (prm.currents) {
-    P.uc[ia] = M.ucb[q] * a + M.ucf[q] * sumt / dtg;
-    P.vc[ia] = M.vcb[q] * a + M.vcf[q] * sumt / dtg;
-  }
-  if (prm.air_density) P.rhoa[ia] = M.rhoab[q] * a + M.rhoaf[q] * sumt / dtg;
-  if (prm.water_density) P.rhow[ia] = M.rhowb[q] * a + M.rhowf[q] * sumt / dtg;
-  P.rhorat[ia] = P.rhoa[ia] / P.rhow[ia];
-  const float ws = fmaxf(P.wspd[ia], 1e-2f);
-  P.wspd[ia] = ws;
-  set_anycurrent(ctl, (prm.isglobal || i < M.N) && (P.uc[ia] != 0.f || P.vc[ia] != 0.f));
-  if (i < M.N) {
-    const int j = M.off + i;
-    float fc = 0.53f * prm.g / ws;
-    if (fc > prm.fprog) fc = prm.fprog;
-    P.fcutoff[j] = fc;
-    const int oc = cutoff_level(prm, fc);
-    P.oc[j] = oc;
-    if (compute_rot) P.oc_rot[j] = oc;
-    P.shelt[j] = shelter_coare35(ws);
-  }
-}
-
-// The same in two halves, for a thread that takes several points (the
-// persistent kernel): prep_load issues every load of a point, prep_finish
-// computes and stores, and prep_points loads all its points before it
-// stores any, so their memory latencies overlap.
+// wet points also oc, oc_rot and the sheltering coefficient), in two halves:
+// prep_load issues every load of a point, prep_finish computes and stores (a
+// load behind a store would wait for the member's pointers to be read again),
+// and prep_points loads all its points before it stores any.
 struct PrepIn {
   int q;
   float w[4];   // uwb, uwf, vwb, vwf; or w[0] = wspd when the winds are fixed
@@ -109,7 +63,7 @@ __device__ __forceinline__ PrepIn prep_load(const Params& prm, const Ptrs& P, co
   return in;
 }
 
-__device__ __forceinline__ void prep_finish(const Params& prm, const Ptrs& P, const Member& M, Ctl* ctl, int i,
+__device__ __forceinline__ bool prep_finish(const Params& prm, const Ptrs& P, const Member& M, Ctl* ctl, int i,
                                             const PrepIn& in, int compute_rot) {
   const float sumt = ctl->sumt, dtg = prm.dtg;
   const float a = 1.f - sumt / dtg;
@@ -142,7 +96,6 @@ __device__ __forceinline__ void prep_finish(const Params& prm, const Ptrs& P, co
   P.rhorat[ia] = rhoa / rhow;
   const float ws = fmaxf(wspd, 1e-2f);
   P.wspd[ia] = ws;
-  set_anycurrent(ctl, (prm.isglobal || i < M.N) && (uc != 0.f || vc != 0.f));
   if (i < M.N) {
     const int j = M.off + i;
     float fc = 0.53f * prm.g / ws;
@@ -153,19 +106,23 @@ __device__ __forceinline__ void prep_finish(const Params& prm, const Ptrs& P, co
     if (compute_rot) P.oc_rot[j] = oc;
     P.shelt[j] = shelter_coare35(ws);
   }
+  return (prm.isglobal || i < M.N) && (uc != 0.f || vc != 0.f);
 }
 
-// Points i0, i0 + stride, ... (U of them, those below M.NM) of one thread.
+// Points i0, i0 + stride, ... (U of them, those below M.NM) of one thread;
+// whether one has a current.
 template <int U>
-__device__ __forceinline__ void prep_points(const Params& prm, const Ptrs& P, const Member& M, Ctl* ctl, int i0,
+__device__ __forceinline__ bool prep_points(const Params& prm, const Ptrs& P, const Member& M, Ctl* ctl, int i0,
                                             int stride, int compute_rot) {
   PrepIn in[U];
 #pragma unroll
   for (int u = 0; u < U; ++u)
     if (i0 + u * stride < M.NM) in[u] = prep_load(prm, P, M, i0 + u * stride);
+  bool cur = false;
 #pragma unroll
   for (int u = 0; u < U; ++u)
-    if (i0 + u * stride < M.NM) prep_finish(prm, P, M, ctl, i0 + u * stride, in[u], compute_rot);
+    if (i0 + u * stride < M.NM) cur |= prep_finish(prm, P, M, ctl, i0 + u * stride, in[u], compute_rot);
+  return cur;
 }
 
 // source(): dts = min(min_i physics_time_step, dtamin, dtg - sumt), the
