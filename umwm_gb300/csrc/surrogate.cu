@@ -10,6 +10,7 @@
 #include <vector>
 
 #include "../../include/umwm_gpu.h"
+#include "host_copy.hpp"
 #include "mlp.hpp"
 #include "surrogate.hpp"
 
@@ -87,6 +88,7 @@ struct State {
   long long timed_steps = 0;
   long long rows_gemm = 0;
   // training batch buffers
+  DevBuf xs;  // f32 rows on their way in (rows_to_bf16), up to COPY_PIECE bytes
   DevBuf bX, bT, Z1, H1, Z2, H2, Yf, dY, dZ2, dZ1, dYt, H2t, dZ2t, H1t, dZ1t, Xt, bidx, loss;
 };
 
@@ -171,6 +173,18 @@ int forward(const bf16* X, int n, bf16* H1, bf16* H2, bf16* Z1, bf16* Z2, float*
     return rc;
   if (Yf) return gemm(H2, S.W3.as<bf16>(), n, FPAD, HID, tc::EPI_F32, Yf, FPAD, w + OFF_B3, nullptr, nullptr, 0, st);
   return gemm(H2, S.W3.as<bf16>(), n, FPAD, HID, tc::EPI_BF16, Ybf, FPAD, w + OFF_B3, nullptr, nullptr, 0, st);
+}
+
+// n rows of FPAD floats from the host as bf16, in pieces through one buffer
+int rows_to_bf16(const float* X, int n, bf16* out) {
+  const int pts = (int)(COPY_PIECE / (FPAD * sizeof(float)));
+  SCU(S.xs.ensure((size_t)std::min(n, pts) * FPAD * sizeof(float)));
+  for (int i = 0; i < n; i += pts) {
+    const size_t cnt = (size_t)std::min(pts, n - i) * FPAD, at = (size_t)i * FPAD;
+    SCU(cudaMemcpyAsync(S.xs.p, X + at, cnt * sizeof(float), cudaMemcpyHostToDevice, S.st));
+    SCU(launch_f32_to_bf16(S.xs.as<float>(), (long)cnt, out + at, S.st));
+  }
+  return UMWM_OK;
 }
 
 int ensure_batch(int B) {
@@ -560,16 +574,18 @@ int umwm_gpu_surrogate_forward(const float* X, int n, float* Y) {
   if (rc) return rc;
   if (!X || !Y || n <= 0) return set_error(UMWM_ERR_ARG, "surrogate_forward: bad arguments");
   if ((rc = ensure_batch(n))) return rc;
-  DevBuf xf;
-  SCU(xf.ensure((size_t)n * FPAD * 4));
-  SCU(cudaMemcpyAsync(xf.p, X, (size_t)n * FPAD * 4, cudaMemcpyHostToDevice, S.st));
-  SCU(launch_f32_to_bf16(xf.as<float>(), (long)n * FPAD, S.bX.as<bf16>(), S.st));
+  if ((rc = rows_to_bf16(X, n, S.bX.as<bf16>()))) return rc;
   if ((rc = forward(S.bX.as<bf16>(), n, S.H1.as<bf16>(), S.H2.as<bf16>(), S.Z1.as<bf16>(), S.Z2.as<bf16>(),
                     S.Yf.as<float>(), nullptr, S.st)))
     return rc;
-  SCU(cudaMemcpyAsync(Y, S.Yf.p, (size_t)n * FPAD * 4, cudaMemcpyDeviceToHost, S.st));
+  const size_t total = (size_t)n * FPAD * sizeof(float);
+  const PageTouch pages(Y, total, COPY_PIECE);  // while the device is at work
+  for (size_t b = 0, c = 0; b < total; b += COPY_PIECE, ++c) {
+    pages.wait(c);
+    SCU(cudaMemcpyAsync(reinterpret_cast<char*>(Y) + b, static_cast<const char*>(S.Yf.p) + b,
+                        std::min(COPY_PIECE, total - b), cudaMemcpyDeviceToHost, S.st));
+  }
   SCU(cudaStreamSynchronize(S.st));
-  xf.release();
   return check_err();
 }
 
@@ -578,18 +594,13 @@ int umwm_gpu_surrogate_grad(const float* X, const float* T, int n, float* loss, 
   if (rc) return rc;
   if (!X || !T || n <= 0 || n % 64) return set_error(UMWM_ERR_ARG, "surrogate_grad: n must be a multiple of 64");
   if ((rc = ensure_batch(n))) return rc;
-  DevBuf xf;
-  SCU(xf.ensure((size_t)n * FPAD * 4));
-  SCU(cudaMemcpyAsync(xf.p, X, (size_t)n * FPAD * 4, cudaMemcpyHostToDevice, S.st));
-  SCU(launch_f32_to_bf16(xf.as<float>(), (long)n * FPAD, S.bX.as<bf16>(), S.st));
-  SCU(cudaMemcpyAsync(xf.p, T, (size_t)n * FPAD * 4, cudaMemcpyHostToDevice, S.st));
-  SCU(launch_f32_to_bf16(xf.as<float>(), (long)n * FPAD, S.bT.as<bf16>(), S.st));
+  if ((rc = rows_to_bf16(X, n, S.bX.as<bf16>()))) return rc;
+  if ((rc = rows_to_bf16(T, n, S.bT.as<bf16>()))) return rc;
   SCU(cudaMemsetAsync(S.loss.p, 0, sizeof(float), S.st));
   if ((rc = backward(n, S.loss.as<float>(), S.st))) return rc;
   if (loss) SCU(cudaMemcpyAsync(loss, S.loss.p, sizeof(float), cudaMemcpyDeviceToHost, S.st));
   if (grad) SCU(cudaMemcpyAsync(grad, S.g.p, NPARAM * 4, cudaMemcpyDeviceToHost, S.st));
   SCU(cudaStreamSynchronize(S.st));
-  xf.release();
   return check_err();
 }
 

@@ -26,6 +26,7 @@
 #include <vector>
 
 #include "../../include/umwm_gpu.h"
+#include "host_copy.hpp"
 #include "host_model.hpp"
 #include "kernels.hpp"
 #include "ncfile.hpp"
@@ -179,6 +180,10 @@ struct Model {
   double kms[K_NK] = {0};
   long long kcnt[K_NK] = {0};
   float *E = nullptr, *ES = nullptr, *TAB = nullptr;
+  // whole points in the reference's order, on their way between E and the host
+  // (state_to_host, set_state_member; one call at a time)
+  float* stage = nullptr;
+  std::mutex stage_mu;
   Tuner tune;
   // persistent substep kernel (option "persistent"): its launch captured in a
   // graph once per launch configuration (pgraph_state 1), or launched
@@ -861,21 +866,60 @@ int init_device(Model& M) {
   return UMWM_OK;
 }
 
+// Points per piece of a spectrum's copy (whole blocks), and the buffer for
+// one: a spectrum-sized buffer per call would need as much again as the
+// spectrum, and its allocation and release took 0.5 ms at 759 MB.
+int stage_points(Model& M, int* pts) {
+  const size_t R = (size_t)M.prm.O * M.prm.P;
+  size_t n = std::max<size_t>(COPY_PIECE / (R * sizeof(float)) / 32 * 32, 32), most = 0;
+  for (const MemberHost& mh : M.mem) most = std::max(most, (size_t)mh.N);
+  n = std::min(n, (most + 31) / 32 * 32);
+  if (!M.stage) CU(M.dev->alloc(&M.stage, n * R, false));
+  *pts = (int)n;
+  return UMWM_OK;
+}
+
 int set_state_member(Model& M, int m, const float* F, const float* ust) {
   const Params& p = M.prm;
   const MemberHost& mh = M.mem[m];
   if (F) {
-    const size_t n = (size_t)p.O * p.P * mh.N;
-    float* tmp = nullptr;
-    CU(cudaMalloc(&tmp, n * 4));
-    cudaError_t e = cudaMemcpy(tmp, F, n * 4, cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = launch_from_ref(p, tmp, M.E, mh.off, mh.N, M.st);
+    std::lock_guard<std::mutex> lk(M.stage_mu);
+    const size_t R = (size_t)p.O * p.P;
+    int pts = 0, rc = stage_points(M, &pts);
+    if (rc) return rc;
+    cudaError_t e = cudaSuccess;
+    for (int i = 0; i < mh.N && e == cudaSuccess; i += pts) {
+      const int n = std::min(pts, mh.N - i);
+      e = cudaMemcpyAsync(M.stage, F + i * R, n * R * sizeof(float), cudaMemcpyHostToDevice, M.st);
+      if (e == cudaSuccess) e = launch_from_ref(p, M.stage, M.E, mh.off + i, n, M.st);
+    }
     if (e == cudaSuccess) e = launch_mss(p, M.P, mh.off, mh.padded, M.st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(M.st);
-    cudaFree(tmp);
+    const cudaError_t es = cudaStreamSynchronize(M.st);  // F is the caller's again, whatever failed
     CU(e);
+    CU(es);
   }
   if (ust) CU(cudaMemcpy(M.P.ustar + mh.off, ust, (size_t)mh.N * 4, cudaMemcpyHostToDevice));
+  return UMWM_OK;
+}
+
+// A spectrum in the device layout (E, or the kept source terms) of a member to
+// the host in the reference's order.
+int state_to_host(Model& M, const MemberHost& mh, const float* src, float* F) {
+  std::lock_guard<std::mutex> lk(M.stage_mu);
+  const size_t R = (size_t)M.prm.O * M.prm.P;
+  int pts = 0, rc = stage_points(M, &pts);
+  if (rc) return rc;
+  const PageTouch pages(F, mh.N * R * sizeof(float), pts * R * sizeof(float));
+  cudaError_t e = cudaSuccess;
+  for (int i = 0, c = 0; i < mh.N && e == cudaSuccess; i += pts, ++c) {
+    const int n = std::min(pts, mh.N - i);
+    e = launch_to_ref(M.prm, src, M.stage, mh.off + i, n, M.st);
+    pages.wait(c);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(F + i * R, M.stage, n * R * sizeof(float), cudaMemcpyDeviceToHost, M.st);
+  }
+  const cudaError_t es = cudaStreamSynchronize(M.st);
+  CU(e);
+  CU(es);
   return UMWM_OK;
 }
 
@@ -1698,13 +1742,11 @@ Model* need_model(bool device) {
 // ---------------------------------------------------------------------------
 // umwm_gpu_get_state_noalloc: the state read-back without device allocation.
 //
-// umwm_gpu_get_state transposes the spectrum into a temporary device buffer as
-// large as the spectrum itself (om*pm*im floats, 4.2 GB on a 1000x1000 grid),
-// allocated and freed on every call.  Some callers cannot do that: a job whose
-// GPU memory is fully committed to an ensemble or to another model's pool
-// allocator (the temporary would not fit, and a failed checkpoint loses the
-// run), or a time-critical coupling loop that must not pay cudaFree's implicit
-// device-wide synchronisation.  This variant streams the transpose through a
+// umwm_gpu_get_state transposes the spectrum through a buffer of up to 32 MiB
+// that the model allocates on first use and keeps.  Some callers cannot do that:
+// a job whose GPU memory is fully committed to an ensemble or to another
+// model's pool allocator (the buffer would not fit, and a failed checkpoint
+// loses the run), or a loop in which no call may allocate.  This variant streams the transpose through a
 // fixed scratch area compiled into the library instead.
 //
 // The scratch is a file-scope __device__ array of NOALLOC_SCRATCH_FLOATS
@@ -1877,18 +1919,11 @@ int umwm_gpu_set_state(const float* F, const float* ust) {
 int umwm_gpu_get_state(float* F, float* ust) {
   Model* M = need_model(true);
   if (!M) return UMWM_ERR_STATE;
-  const Params& p = M->prm;
   const MemberHost& mh = M->mem[M->sel];
   CU(cudaStreamSynchronize(M->st));
   if (F) {
-    const size_t n = (size_t)p.O * p.P * mh.N;
-    float* tmp = nullptr;
-    CU(cudaMalloc(&tmp, n * 4));
-    cudaError_t e = launch_to_ref(p, M->E, tmp, mh.off, mh.N, M->st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(M->st);
-    if (e == cudaSuccess) e = cudaMemcpy(F, tmp, n * 4, cudaMemcpyDeviceToHost);
-    cudaFree(tmp);
-    CU(e);
+    const int rc = state_to_host(*M, mh, M->E, F);
+    if (rc) return rc;
   }
   if (ust) CU(cudaMemcpy(ust, M->P.ustar + mh.off, (size_t)mh.N * 4, cudaMemcpyDeviceToHost));
   return UMWM_OK;
@@ -2005,14 +2040,7 @@ int umwm_gpu_get_field(const char* name, float* out, long n) {
     const size_t cnt = (size_t)M->prm.O * M->prm.P * mh.N;
     if (need((long)cnt)) return UMWM_ERR_ARG;
     const float* src = s == "ssin" ? M->P.src_sin : s == "sds" ? M->P.src_sds : M->P.src_snl;
-    float* tmp = nullptr;
-    CU(cudaMalloc(&tmp, cnt * 4));
-    cudaError_t e = launch_to_ref(M->prm, src, tmp, mh.off, mh.N, M->st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(M->st);
-    if (e == cudaSuccess) e = cudaMemcpy(out, tmp, cnt * 4, cudaMemcpyDeviceToHost);
-    cudaFree(tmp);
-    CU(e);
-    return UMWM_OK;
+    return state_to_host(*M, mh, src, out);
   }
   if (s == "ar") return wet_host(H.ar);
   if (s == "oneovar") return wet_host(H.oneovar);
@@ -2099,9 +2127,10 @@ int umwm_gpu_get_field(const char* name, float* out, long n) {
   if (s == "us" || s == "vs") {
     if (need((long)H.lm * N)) return UMWM_ERR_ARG;
     const float* src = s == "us" ? P.us : P.vs;
-    for (int l = 0; l < H.lm; ++l)
-      CU(cudaMemcpy(out + (size_t)l * N, src + (size_t)l * M->prm.ldN + mh.off, (size_t)N * 4,
-                    cudaMemcpyDeviceToHost));
+    // one strided copy (a copy per depth: 0.9 ms for the 42 depths of 171 points)
+    if (H.lm > 0 && N > 0)
+      CU(cudaMemcpy2D(out, (size_t)N * 4, src + mh.off, (size_t)M->prm.ldN * 4, (size_t)N * 4, H.lm,
+                      cudaMemcpyDeviceToHost));
     return UMWM_OK;
   }
   Ctl c;
