@@ -122,9 +122,9 @@ int umwm_gpu_set_state(const float* F, const float* ust);
 /* Same output as umwm_gpu_get_state, for callers that cannot allocate device
  * memory at that moment: a job whose GPU memory is fully committed to an
  * ensemble or a pool allocator, or a loop in which no call may allocate.  The
- * first umwm_gpu_get_state or
- * umwm_gpu_set_state of a model allocates a buffer of up to 32 MiB that the
- * model keeps; this variant allocates nothing and streams the spectrum to F through a fixed
+ * first umwm_gpu_get_state or umwm_gpu_set_state of a model allocates a buffer
+ * of up to 32 MiB that the model keeps; this variant allocates nothing and
+ * streams the spectrum to F through a fixed
  * 16 MiB scratch array compiled into the library (held on every GPU that
  * loads the library until the process exits), in chunks of whole wet points,
  * all on the model's stream.  A point's spectrum larger than the scratch

@@ -47,6 +47,7 @@ __global__ void __launch_bounds__(W * 32, MINB) k_advect(const Params prm, const
   extern __shared__ __align__(128) float dsm[];
   __shared__ float4 dirs[NP / 4 * DIR_ROWS], cw[NP / 4 * 32];
   dir_fill<NP>(prm, reinterpret_cast<float*>(dirs));  // (advect_body's barrier)
+  wait_previous(prm);
   advect_body<NP, CURV, CNT, false>(prm, P, blockIdx.x, adv_smem_u32(dirs), cw, dsm, dsm + adv_red_floats(prm.O));
   // the block of a member's print point (its first block without one) writes
   // the member's screen line and counts the substep; a kernel of its own took
@@ -65,8 +66,7 @@ static cudaError_t go(const Params& prm, const Ptrs& P, int warps, cudaStream_t 
   const cudaError_t e = allow_smem((const void*)k_advect<NP, CURV, W, MINB, CNT>,
                                    (adv_red_floats(MAX_OM) + (size_t)W * adv_ring_floats<NP>()) * sizeof(float), done);
   if (e != cudaSuccess) return e;
-  k_advect<NP, CURV, W, MINB, CNT><<<prm.Ntot / 32, warps * 32, smem, st>>>(prm, P);
-  return cudaGetLastError();
+  return launch_chained(k_advect<NP, CURV, W, MINB, CNT>, prm.Ntot / 32, warps * 32, smem, st, prm, P);
 }
 
 // prm.adv_groups4: 16 warps per block (8 where the blocks are more than one

@@ -15,6 +15,7 @@ namespace umwm {
 // clamp wspd, rhorat; per wet point the cut-off index oc and the
 // sheltering coefficient (umwm_source_functions.F90:52).
 __global__ void k_prep(const Params prm, const Ptrs P, int compute_rot) {
+  let_next_start(prm);
   const Member& M = prm.mem[blockIdx.y];
   Ctl* ctl = M.ctl;
   if (ctl->done) return;
@@ -60,6 +61,7 @@ __device__ __forceinline__ void fill_cs(const Params& prm, float* cs) {
 // factor C1*Hs (Hs < 3 m) or C1*3 (umwm_source_functions.F90:108-153).
 __global__ void __launch_bounds__(MW * 32) k_sice(const Params prm, const Ptrs P) {
   __shared__ float part[MW][32];
+  wait_previous(prm);
   const Member& M = prm.mem[prm.tile_mem[(blockIdx.x * 32) / TILE]];
   BlockPoint b;
   if (M.ctl->done || !block_point(M, b)) return;
@@ -453,8 +455,7 @@ cudaError_t launch_prep(const Params& prm, const Ptrs& P, int compute_rot, int m
   return cudaGetLastError();
 }
 cudaError_t launch_sice(const Params& prm, const Ptrs& P, cudaStream_t st) {
-  k_sice<<<prm.Ntot / 32, MW * 32, 0, st>>>(prm, P);
-  return cudaGetLastError();
+  return launch_chained(k_sice, prm.Ntot / 32, MW * 32, 0, st, prm, P);
 }
 cudaError_t launch_diag(const Params& prm, const Ptrs& P, cudaStream_t st) {
   k_diag<<<prm.Ntot / 32, MW * 32, 0, st>>>(prm, P);

@@ -65,6 +65,7 @@ __global__ void __launch_bounds__(W * 32, MINB)
   __shared__ float4 dirs[NP / 4 * DIR_ROWS], cw[NP / 4 * 32];
   __shared__ __align__(8) unsigned long long mbar[TMA ? 2 * W : 1];
   dir_fill<NP>(prm, reinterpret_cast<float*>(dirs));  // (phys_body's barrier)
+  wait_previous(prm);
   phys_body<NP, TMA>(prm, P, compute_rot, blockIdx.x, adv_smem_u32(dirs), cw, red, dsm, adv_smem_u32(mbar));
   if constexpr (!END) return;
   // thread 0 of each block wrote the block's minimum and maximum
@@ -79,6 +80,7 @@ __global__ void __launch_bounds__(W * 32, MINB)
   dts_end(prm, P, compute_rot, end);
 }
 __global__ void k_dts(const Params prm, const Ptrs P, int compute_rot, const SubstepEnd end) {
+  wait_previous(prm);
   dts_end(prm, P, compute_rot, end);
 }
 
@@ -92,8 +94,7 @@ static cudaError_t go_phys(const Params& prm, const Ptrs& P, int compute_rot, co
         allow_smem((const void*)k_phys<NP, W, MINB, TMA, END>, (size_t)W * 2 * NP * 32 * sizeof(float), done);
     if (e != cudaSuccess) return e;
   }
-  k_phys<NP, W, MINB, TMA, END><<<prm.Ntot / 32, warps * 32, smem, st>>>(prm, P, compute_rot, end);
-  return cudaGetLastError();
+  return launch_chained(k_phys<NP, W, MINB, TMA, END>, prm.Ntot / 32, warps * 32, smem, st, prm, P, compute_rot, end);
 }
 
 // prm.groups4_phys: 16 warps per block (8 where the blocks are more than one
@@ -122,13 +123,13 @@ __global__ void __launch_bounds__(WMAX * 32, MINB) k_integ(const Params prm, con
   dir_fill<NP>(prm, reinterpret_cast<float*>(dirs));
   __syncthreads();
   const int w = threadIdx.x >> 5;
+  wait_previous(prm);
   integ_body<NP>(prm, P, adv_smem_u32(dirs), cw + (w / NG) * (NP / 4 * 32), blockIdx.x, w, nc);
 }
 
 template <int NP, int WMAX, int MINB>
 static cudaError_t go_integ(const Params& prm, const Ptrs& P, int nc, cudaStream_t st) {
-  k_integ<NP, WMAX, MINB><<<prm.Ntot / 32, 32 * nc * (NP / integ_dirs<NP>()), 0, st>>>(prm, P, nc);
-  return cudaGetLastError();
+  return launch_chained(k_integ<NP, WMAX, MINB>, prm.Ntot / 32, 32 * nc * (NP / integ_dirs<NP>()), 0, st, prm, P, nc);
 }
 
 // prm.groups4: the levels of a block in several chunks (small models: the
@@ -166,8 +167,7 @@ cudaError_t launch_source_phys(const Params& prm, const Ptrs& P, int compute_rot
   UMWM_ALL_NP(launch_phys_np, prm, P, compute_rot, end, st)
 }
 cudaError_t launch_dts(const Params& prm, const Ptrs& P, int compute_rot, const SubstepEnd& end, cudaStream_t st) {
-  k_dts<<<1, 128, 0, st>>>(prm, P, compute_rot, end);
-  return cudaGetLastError();
+  return launch_chained(k_dts, 1, 128, 0, st, prm, P, compute_rot, end);
 }
 cudaError_t launch_source_integ(const Params& prm, const Ptrs& P, cudaStream_t st) {
   UMWM_ALL_NP(launch_integ_np, prm, P, st)

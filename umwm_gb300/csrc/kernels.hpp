@@ -19,6 +19,25 @@ inline cudaError_t allow_smem(const void* f, size_t bytes, std::atomic<unsigned 
   return e;
 }
 
+// Launch of a substep's kernel behind another one on the stream: its blocks may
+// start while the last of the kernel before are at work, up to
+// wait_previous(), so that the launch and the kernel's set-up are off
+// the chain of a substep's kernels.
+template <typename... K, typename... A>
+cudaError_t launch_chained(void (*f)(K...), int grid, int block, size_t smem, cudaStream_t st, const A&... a) {
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t c{};
+  c.gridDim = dim3((unsigned)grid);
+  c.blockDim = dim3((unsigned)block);
+  c.dynamicSmemBytes = smem;
+  c.stream = st;
+  c.attrs = &at;
+  c.numAttrs = 1;
+  return cudaLaunchKernelEx(&c, f, a...);
+}
+
 bool supported_pm(int pm);
 cudaError_t launch_prep(const Params& prm, const Ptrs& P, int compute_rot, int max_nm, cudaStream_t st);
 cudaError_t launch_sice(const Params& prm, const Ptrs& P, cudaStream_t st);
