@@ -339,6 +339,7 @@ __device__ __forceinline__ void advect_body(const Params& prm, const Ptrs& P, in
     rl_[0] = tx * kdk;
     rl_[32] = ty * kdk;
     rl_[64] = hk * (m0.x + m0.y);
+    if (prm.ice_possible) P.ehs[((size_t)blk * O + o) * 32 + lane] = kdk * (m0.x + m0.y);
     rl_[96] = hk * (m1.x + m1.y);
     rl_[128] = hk * (m2.x + m2.y);
     if (o == O - 1) {

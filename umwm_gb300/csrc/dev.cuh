@@ -167,7 +167,7 @@ struct Global {
   int bar_err;
   // time block 0 of the persistent kernel spent in each stage, up to and
   // including the barrier that ends it (globaltimer ns, accumulated over
-  // launches until read): forcing, sea ice, dts pre-pass, dts, integration,
+  // launches until read): forcing, (none), dts pre-pass, dts, integration,
   // propagation, screen
   unsigned long long stage_ns[8];
 };
@@ -190,6 +190,7 @@ struct Ptrs {
   float* fcutoff;
   float* phys;      // physics_time_step
   float* sice_v;    // per-point sea-ice attenuation factor (0 when no ice)
+  float* ehs;       // models with sea ice: a level's sum of e times k dk, [NB][O][32], kept with MSS
   // all-point arrays, member m at [nmoff, nmoff+NM) (land included; wet
   // points first, in the member's unrolled order)
   float *wspd, *wdir, *uc, *vc, *rhoa, *rhow, *rhorat, *fice;

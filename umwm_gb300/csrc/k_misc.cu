@@ -1,6 +1,5 @@
-// Per-substep forcing and cut-off kernel, the sea-ice Hs, and the
-// once-per-output kernels: diag, Stokes drift, stress('ocn') and the spectrum
-// layout transposes.
+// Per-substep forcing and cut-off kernel, and the once-per-output kernels:
+// diag, Stokes drift, stress('ocn') and the spectrum layout transposes.
 #include <algorithm>
 #include <cfloat>
 
@@ -25,14 +24,12 @@ __global__ void k_prep(const Params prm, const Ptrs P, int compute_rot) {
   set_anycurrent(ctl, cur);
 }
 
-// The once-per-interval kernels below and the sea-ice wave height share one
-// mapping: a CTA owns a block of 32 points (lane = point), its MW warps take
+// The once-per-interval kernels below share one mapping: a CTA owns a block of 32 points (lane = point), its MW warps take
 // every MW-th frequency level and read four directions of 32 points per
 // access, and the warps' partial sums meet in shared memory.  One thread per
 // point walked 1332 bins in a chain of dependent loads: 94 us at 171 points
 // and 543 us at 305 k for the diagnostics, 270 and 1140 us for the Stokes
-// drift, 74 us per substep at 13 k points for the sea-ice wave height.  So
-// split: 18 and 503 us, 26 and 493 us, and 23 us (small models wait on the
+// drift.  So split: 18 and 503 us, 26 and 493 us (small models wait on the
 // levels' chain; at 305 k points the 1.6 GB spectrum is read at 3.2 TB/s, the
 // rest being the level sums' instructions).
 constexpr int MW = 8;
@@ -55,25 +52,6 @@ __device__ __forceinline__ void fill_cs(const Params& prm, float* cs) {
     cs[(p >> 2) * 8 + (p & 3)] = prm.cth[p];
     cs[(p >> 2) * 8 + 4 + (p & 3)] = prm.sth[p];
   }
-}
-
-// s_ice: significant wave height where fice > fice_lth and the attenuation
-// factor C1*Hs (Hs < 3 m) or C1*3 (umwm_source_functions.F90:108-153).
-__global__ void __launch_bounds__(MW * 32) k_sice(const Params prm, const Ptrs P) {
-  __shared__ float part[MW][32];
-  wait_previous(prm);
-  const Member& M = prm.mem[prm.tile_mem[(blockIdx.x * 32) / TILE]];
-  BlockPoint b;
-  if (M.ctl->done || !block_point(M, b)) return;
-  const bool ice = b.valid && P.fice[apt(M, b.valid ? b.j : M.ghost)] > prm.fice_lth;
-  float h = 0.f;
-  if (__any_sync(0xffffffffu, ice)) h = sice_levels(prm, P, b.j, b.w, MW);
-  part[b.w][b.lane] = h;
-  __syncthreads();
-  if (b.w != 0 || !b.valid) return;
-  h = 0.f;
-  for (int i = 0; i < MW; ++i) h += part[i][b.lane];
-  P.sice_v[b.j] = ice ? sice_factor(prm, h) : 0.f;
 }
 
 // diag, umwm_physics.F90:89-205.  A level's direction sums are formed first
@@ -302,6 +280,7 @@ __global__ void __launch_bounds__(128) k_mss(const Params prm, const Ptrs P, int
     }
     const float hk = P.TAB[tidx(prm, o, T_K3DK, j)] * (0.5f * prm.dth);
     v[o * 96 + lane] = hk * a;
+    if (prm.ice_possible) P.ehs[((size_t)blk * prm.O + o) * 32 + lane] = P.TAB[tidx(prm, o, T_KDK, j)] * a;
     v[o * 96 + 32 + lane] = hk * b;
     v[o * 96 + 64 + lane] = hk * c;
   }
@@ -453,9 +432,6 @@ cudaError_t launch_prep(const Params& prm, const Ptrs& P, int compute_rot, int m
   dim3 grid(grid_for(max_nm, 256), prm.nmem);
   k_prep<<<grid, 256, 0, st>>>(prm, P, compute_rot);
   return cudaGetLastError();
-}
-cudaError_t launch_sice(const Params& prm, const Ptrs& P, cudaStream_t st) {
-  return launch_chained(k_sice, prm.Ntot / 32, MW * 32, 0, st, prm, P);
 }
 cudaError_t launch_diag(const Params& prm, const Ptrs& P, cudaStream_t st) {
   k_diag<<<prm.Ntot / 32, MW * 32, 0, st>>>(prm, P);

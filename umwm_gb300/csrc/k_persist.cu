@@ -1,7 +1,7 @@
 // Persistent substep kernel: the inner dynamic-dts loop of umwm_run
 // (umwm_top.F90:97-150) for every member of a model in one cooperative
 // launch.  Each CTA loops over substeps; within a substep it takes the
-// stages in order (forcing interpolation, [sea-ice Hs], the dts pre-pass,
+// stages in order (forcing interpolation, the dts pre-pass,
 // dts, the integration, propagation + refraction + stress, the screen line),
 // working through the stage's tiles grid-stride, with a grid-wide barrier
 // between stages.  The stage bodies are those of the per-stage kernels
@@ -124,10 +124,6 @@ __global__ void __launch_bounds__(128, UMWM_PERSIST_MINB)
   for (int it = 0; it < budget; ++it) {
     forcing_stage(prm, P, nb, compute_rot);
     if (!bar_s(0)) return;
-    if (prm.ice_possible) {
-      for (int j = blockIdx.x * 128 + threadIdx.x; j < prm.Ntot; j += nb * 128) sice_point(prm, P, j, 8);
-      if (!bar_s(1)) return;
-    }
     for (int v = blockIdx.x; v < nvb; v += nb) {
       phys_body<NP, 0>(prm, P, compute_rot, v, dirs, cw, phys_s, nullptr, 0u);
       __syncthreads();  // the next block reuses the maxima

@@ -40,7 +40,6 @@ cudaError_t launch_chained(void (*f)(K...), int grid, int block, size_t smem, cu
 
 bool supported_pm(int pm);
 cudaError_t launch_prep(const Params& prm, const Ptrs& P, int compute_rot, int max_nm, cudaStream_t st);
-cudaError_t launch_sice(const Params& prm, const Ptrs& P, cudaStream_t st);
 // What follows the dts pre-pass's last block: dts, dtr and sumt of every
 // member, and in a graph the count of the substep and the condition of its
 // while node (another substep while a member is inside the dtg and the budget

@@ -1,5 +1,5 @@
 // Device bodies of the per-substep control kernels (forcing interpolation,
-// dts/dtr, sea-ice Hs, screen line), shared by their per-stage kernels in
+// dts/dtr, screen line), shared by their per-stage kernels in
 // k_misc.cu and the persistent substep kernel.
 #pragma once
 #include <cfloat>
@@ -32,10 +32,26 @@ __device__ __forceinline__ void set_anycurrent(Ctl* ctl, bool cur) {
 // prep_load issues every load of a point, prep_finish computes and stores (a
 // load behind a store would wait for the member's pointers to be read again),
 // and prep_points loads all its points before it stores any.
+// s_ice: the attenuation factor C1 Hs, Hs at most 3 m, where fice > fice_lth
+// (umwm_source_functions.F90:108-153), from the levels' energy sums that the
+// propagation leaves.  (A pass over the spectrum for them took 23 us a substep
+// at 13 k points, beside 185 for the rest; summed in the propagation's tail
+// they cost it 9 to 15 us; so, the forcing 5 and the propagation 2.)
+__device__ __forceinline__ float sice_factor(const Params& prm, const Ptrs& P, float fice, int j) {
+  if (!(fice > prm.fice_lth)) return 0.f;
+  const float* v = P.ehs + (size_t)(j >> 5) * prm.O * 32 + (j & 31);
+  float h = 0.f;
+#pragma unroll 8
+  for (int o = 0; o < prm.O; ++o) h += v[o * 32];
+  h = 4.f * sqrtf(h * prm.dth);
+  const float C1 = -5.35e-6f;
+  return (h < 3.f) ? C1 * h : C1 * 3.f;
+}
+
 struct PrepIn {
   int q;
   float w[4];   // uwb, uwf, vwb, vwf; or w[0] = wspd when the winds are fixed
-  float fi[2];  // ficeb, ficef
+  float fi[2];  // ficeb, ficef; or fi[0] = fice when fixed
   float c[4];   // ucb, ucf, vcb, vcf; or c[0], c[1] = uc, vc when fixed
   float ra[2];  // rhoab, rhoaf; or ra[0] = rhoa when fixed
   float rw[2];  // rhowb, rhowf; or rw[0] = rhow when fixed
@@ -51,6 +67,7 @@ __device__ __forceinline__ PrepIn prep_load(const Params& prm, const Ptrs& P, co
     in.w[0] = P.wspd[ia];
   }
   if (prm.seaice) in.fi[0] = M.ficeb[q], in.fi[1] = M.ficef[q];
+  else if (prm.ice_possible) in.fi[0] = P.fice[ia];
   if (prm.currents) {
     in.c[0] = M.ucb[q], in.c[1] = M.ucf[q], in.c[2] = M.vcb[q], in.c[3] = M.vcf[q];
   } else {
@@ -82,7 +99,8 @@ __device__ __forceinline__ bool prep_finish(const Params& prm, const Ptrs& P, co
     wspd = sqrtf(uw * uw + vw * vw);
     P.wdir[ia] = atan2f(vw, uw);
   }
-  if (prm.seaice) P.fice[ia] = in.fi[0] * a + in.fi[1] * sumt / dtg;
+  float fice = in.fi[0];
+  if (prm.seaice) P.fice[ia] = fice = in.fi[0] * a + in.fi[1] * sumt / dtg;
   float uc = in.c[0], vc = in.c[1];
   if (prm.currents) {
     uc = in.c[0] * a + in.c[1] * sumt / dtg;
@@ -105,6 +123,7 @@ __device__ __forceinline__ bool prep_finish(const Params& prm, const Ptrs& P, co
     P.oc[j] = oc;
     if (compute_rot) P.oc_rot[j] = oc;
     P.shelt[j] = shelter_coare35(ws);
+    if (prm.ice_possible) P.sice_v[j] = sice_factor(prm, P, fice, j);
   }
   return (prm.isglobal || i < M.N) && (uc != 0.f || vc != 0.f);
 }
@@ -162,42 +181,6 @@ __device__ __forceinline__ int dts_body(const Params& prm, const Ptrs& P, int co
   left = __syncthreads_count(left > 0) ? 1 : 0;  // any member left in this block
   if (threadIdx.x == 0) P.glob->not_done = left;
   return left;
-}
-
-// s_ice (umwm_source_functions.F90:108-153): the energy sum of the levels
-// o0, o0 + step, ... of point j, and the attenuation factor of the whole sum
-// (C1 Hs, Hs at most 3 m).
-__device__ __forceinline__ float sice_levels(const Params& prm, const Ptrs& P, int j, int o0, int step) {
-  float h = 0.f;
-  for (int o = o0; o < prm.O; o += step) {
-    const float4* r = reinterpret_cast<const float4*>(P.E + sidx(prm, o, 0, j));
-    float s = 0.f;
-#pragma unroll 3
-    for (int q = 0; q < prm.P / 4; ++q) {
-      const float4 e = r[q * 32];
-      s += (e.x + e.y) + (e.z + e.w);
-    }
-    h = fmaf(s, P.TAB[tidx(prm, o, T_KDK, j)], h);
-  }
-  return h;
-}
-__device__ __forceinline__ float sice_factor(const Params& prm, float h) {
-  h = 4.f * sqrtf(h * prm.dth);
-  const float C1 = -5.35e-6f;
-  return (h < 3.f) ? C1 * h : C1 * 3.f;
-}
-// the same by one thread, its sum in the parts of `parts` warps (the
-// persistent kernel: the same bits as k_sice)
-__device__ __forceinline__ void sice_point(const Params& prm, const Ptrs& P, int j, int parts) {
-  const Member& M = prm.mem[prm.tile_mem[j / TILE]];
-  if (j >= M.ghost || M.ctl->done) return;
-  float sv = 0.f;
-  if (P.fice[apt(M, j)] > prm.fice_lth) {
-    float h = 0.f;
-    for (int i = 0; i < parts; ++i) h += sice_levels(prm, P, j, i, parts);
-    sv = sice_factor(prm, h);
-  }
-  P.sice_v[j] = sv;
 }
 
 // Screen line of member m at its print point (umwm_top.F90:143-148,

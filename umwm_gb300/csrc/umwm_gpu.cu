@@ -40,6 +40,8 @@ Inputs g_inputs;
 int g_device = -1;  // set_option("device", n) before initialize
 
 // Per-kernel CUDA-event timing on the launching stream (option "kernel_timing").
+// The sea-ice wave height and the screen line are parts of other kernels; their
+// statistics stay 0.
 enum KName { K_PREP, K_SICE, K_PHYS, K_DTS, K_INTEG, K_ADVECT, K_DIAG, K_SCREEN, K_STOKES, K_NK };
 const char* const KNAMES[K_NK] = {"prep", "sice", "phys", "dts", "integ", "advect", "diag", "screen", "stokes"};
 
@@ -705,6 +707,7 @@ int init_device(Model& M) {
   for (const MemberHost& mh : M.mem)
     if ((rc = upload_tables(M, mh))) return rc;
   CU(D.alloc(&P.MSS, (size_t)p.O * 3 * ldN, true));
+  if (p.ice_possible) CU(D.alloc(&P.ehs, (size_t)p.O * ldN, true));
   // per-point arrays in the common index space
   auto upload_i = [&](const int** dst, std::vector<int>(HostModel::*field), bool aliased) -> int {
     std::vector<int> h(ldN, 0);
@@ -1410,7 +1413,7 @@ int ensure_ocn(Model& M) {
   return UMWM_OK;
 }
 
-// Enqueue the launches of one substep: prep, [sice], phys, [dts], integ,
+// Enqueue the launches of one substep: prep, phys, [dts], integ,
 // advect (with the screen line), [diag on the first substep of a run].  `loop`:
 // the while node of the graph that is being captured.
 int enqueue_substep(Model& M, int compute_rot, int first, bool diag, const cudaGraphConditionalHandle* loop = nullptr) {
@@ -1418,7 +1421,6 @@ int enqueue_substep(Model& M, int compute_rot, int first, bool diag, const cudaG
   const Ptrs& P = M.P;
   const SubstepEnd end{first, dts_fused(prm) ? 1 : 0, loop ? 1 : 0, loop ? *loop : 0};
   CU(timed(M, K_PREP, [&] { return launch_prep(prm, P, compute_rot, M.max_nm, M.st); }));
-  if (prm.ice_possible) CU(timed(M, K_SICE, [&] { return launch_sice(prm, P, M.st); }));
   CU(tuned(M, TK_PHYS, K_PHYS, [&] { return launch_source_phys(prm, P, compute_rot, end, M.st); }));
   if (!end.fused) CU(timed(M, K_DTS, [&] { return launch_dts(prm, P, compute_rot, end, M.st); }));
   int rc;
@@ -1439,7 +1441,7 @@ int enqueue_substep(Model& M, int compute_rot, int first, bool diag, const cudaG
 }
 
 int substep_launches(const Model& M, bool diag) {
-  return 4 + (dts_fused(M.prm) ? 0 : 1) + (M.prm.ice_possible ? 1 : 0) + (diag ? 1 : 0);
+  return 4 + (dts_fused(M.prm) ? 0 : 1) + (diag ? 1 : 0);
 }
 
 int substep(Model& M) {
