@@ -50,7 +50,7 @@ __device__ __forceinline__ void adv_sts(uint32_t a, float4 v) {
 // is cut to 0 (option "count_cut"; a separate instance so that the plain one
 // carries no counter).  COH: E* is read through L2 only, for a persistent
 // kernel in which the same launch wrote it.  red, ring: shared memory (adv_red_floats, adv_ring_floats per warp).
-template <int NP, bool CURV, bool CNT, bool COH>
+template <int NP, bool CURV, bool CNT, bool COH, bool AHEAD>
 __device__ __forceinline__ void advect_body(const Params& prm, const Ptrs& P, int blk, uint32_t dirs, float4* cw,
                                             float* red, float* ring) {
   constexpr int NQ = NP / 4, S = adv_stages<NP>();
@@ -175,30 +175,51 @@ __device__ __forceinline__ void advect_body(const Params& prm, const Ptrs& P, in
     elast = lde(r + poff(NP - 1));
   }
 
+  // AHEAD: a level's table values, read during the last quad of the level
+  // before (their latency was a sixth of the kernel's stalls: 1176 -> 1152 us
+  // at 305 k points, 511 -> 498 at 144 k); the forms of 128 registers read
+  // them in place, since the 15 registers would spill there
+  struct { float cp0, kdk, fkovg, k3, l2z, cpv, cg, cgE, cgW, cgN, cgS, cpE, cpW, cpN, cpS; } T;
+  auto tab = [&](int o) {
+    if (o >= O) return;
+    const unsigned to = o * tstride;
+    T.cp0 = __ldg(tO + to + T_CP0 * 32), T.kdk = __ldg(tO + to + T_KDK * 32);
+    T.fkovg = __ldg(tO + to + T_FKOVG * 32), T.k3 = __ldg(tO + to + T_K3DK * 32);
+    T.l2z = __ldg(tO + to + T_LOGL2Z * 32), T.cpv = __ldg(tV + to);
+    if (o < ocw) {
+      T.cg = __ldg(tO + to + T_CG0 * 32);
+      T.cgE = __ldg(tE + to + T_CG0 * 32), T.cgW = __ldg(tW + to + T_CG0 * 32);
+      T.cgN = __ldg(tN + to + T_CG0 * 32), T.cgS = __ldg(tS + to + T_CG0 * 32);
+      T.cpE = __ldg(tE + to + T_CP0 * 32), T.cpW = __ldg(tW + to + T_CP0 * 32);
+      T.cpN = __ldg(tN + to + T_CP0 * 32), T.cpS = __ldg(tS + to + T_CP0 * 32);
+    }
+  };
+  if (AHEAD) tab(w);
   for (int o = w; o < O; o += nw) {
     pf(o + PFD * nw);
     const unsigned lo = o * lstride, to = o * tstride;
+    auto tv = [&](float ahead, const float* t) { return AHEAD ? ahead : __ldg(t + to); };
     float* const Eo = P.E + ro + lo;
     const bool prog = o < oc, refr = prog && o < ocr;
     const bool anyp = o < ocw, anyr = __any_sync(0xffffffffu, refr);
-    const float cp0 = __ldg(tO + to + T_CP0 * 32), kdk = __ldg(tO + to + T_KDK * 32);
-    const float fkovg = __ldg(tO + to + T_FKOVG * 32), hk = __ldg(tO + to + T_K3DK * 32) * (0.5f * prm.dth);
-    const float U = fmaf(wi.ustar25, __ldg(tO + to + T_LOGL2Z * 32), wi.wspd);
-    const float icp = 1.f / __ldg(tV + to);
+    const float cp0 = tv(T.cp0, tO + T_CP0 * 32), kdk = tv(T.kdk, tO + T_KDK * 32);
+    const float fkovg = tv(T.fkovg, tO + T_FKOVG * 32), hk = tv(T.k3, tO + T_K3DK * 32) * (0.5f * prm.dth);
+    const float U = fmaf(wi.ustar25, tv(T.l2z, tO + T_LOGL2Z * 32), wi.wspd);
+    const float icp = 1.f / tv(T.cpv, tV);
     const float2 U2 = f2(U), ncp = f2(-cp0), nuc = f2(-uci), nvc = f2(-vci);
     // above the cut-off Sin is cut at 0 (the NaN-keeping maximum with -inf keeps it below)
     const float slo = prog ? __int_as_float(0xff800000) : 0.f;
     float DE = 0.f, DW = 0.f, DN = 0.f, DS = 0.f, alc = 0.f, bec = 0.f;
     if (anyp) {
-      const float cgi = __ldg(tO + to + T_CG0 * 32);
-      DE = 2.f * (cgi + __ldg(tE + to + T_CG0 * 32)) * dye;
-      DW = 2.f * (cgi + __ldg(tW + to + T_CG0 * 32)) * dyw;
-      DN = 2.f * (cgi + __ldg(tN + to + T_CG0 * 32)) * dxn;
-      DS = 2.f * (cgi + __ldg(tS + to + T_CG0 * 32)) * dxs;
+      const float cgi = tv(T.cg, tO + T_CG0 * 32);
+      DE = 2.f * (cgi + tv(T.cgE, tE + T_CG0 * 32)) * dye;
+      DW = 2.f * (cgi + tv(T.cgW, tW + T_CG0 * 32)) * dyw;
+      DN = 2.f * (cgi + tv(T.cgN, tN + T_CG0 * 32)) * dxn;
+      DS = 2.f * (cgi + tv(T.cgS, tS + T_CG0 * 32)) * dxs;
     }
     if (anyr) {
-      const float gx = 0.5f * (__ldg(tE + to + T_CP0 * 32) - __ldg(tW + to + T_CP0 * 32));
-      const float gy = 0.5f * (__ldg(tN + to + T_CP0 * 32) - __ldg(tS + to + T_CP0 * 32));
+      const float gx = 0.5f * (tv(T.cpE, tE + T_CP0 * 32) - tv(T.cpW, tW + T_CP0 * 32));
+      const float gy = 0.5f * (tv(T.cpN, tN + T_CP0 * 32) - tv(T.cpS, tS + T_CP0 * 32));
       alc = gx * odx;
       bec = -(gy * ody);
     }
@@ -219,6 +240,7 @@ __device__ __forceinline__ void advect_body(const Params& prm, const Ptrs& P, in
 #pragma unroll
     for (int q = 0; q < NQ; ++q) {
       const int p = 4 * q;
+      if (AHEAD && q + 1 == NQ) tab(o + nw);
       adv_wait<S - 2>();  // this quad's rows have landed
       const uint32_t d = rg + (uint32_t)(q % S) * 3072u;
       float4 ef4 = adv_lds(d + 512);  // e below the cut-off, ef above

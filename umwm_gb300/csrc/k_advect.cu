@@ -48,7 +48,7 @@ __global__ void __launch_bounds__(W * 32, MINB) k_advect(const Params prm, const
   __shared__ float4 dirs[NP / 4 * DIR_ROWS], cw[NP / 4 * 32];
   dir_fill<NP>(prm, reinterpret_cast<float*>(dirs));  // (advect_body's barrier)
   wait_previous(prm);
-  advect_body<NP, CURV, CNT, false>(prm, P, blockIdx.x, adv_smem_u32(dirs), cw, dsm, dsm + adv_red_floats(prm.O));
+  advect_body<NP, CURV, CNT, false, (MINB > 2)>(prm, P, blockIdx.x, adv_smem_u32(dirs), cw, dsm, dsm + adv_red_floats(prm.O));
   // the block of a member's print point (its first block without one) writes
   // the member's screen line and counts the substep; a kernel of its own took
   // 8 to 14 us a substep, this 0 to 2 us

@@ -134,7 +134,7 @@ __global__ void __launch_bounds__(128, UMWM_PERSIST_MINB)
     for (int u = blockIdx.x * 4 + warp; u < nvb * NG; u += nb * 4) integ_body<NP>(prm, P, dirs, reinterpret_cast<float4*>(dsm) + warp * (NP / 4 * 32), u / NG, u % NG, 1);
     if (!bar_s(4)) return;
     for (int v = blockIdx.x; v < nvb; v += nb) {
-      advect_body<NP, CURV, false, true>(prm, P, v, dirs, cw, dsm, dsm + adv_red_floats(prm.O));
+      advect_body<NP, CURV, false, true, false>(prm, P, v, dirs, cw, dsm, dsm + adv_red_floats(prm.O));
       __syncthreads();  // the next block reuses the sums
     }
     if (!bar_s(5)) return;
