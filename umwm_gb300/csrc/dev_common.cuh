@@ -164,6 +164,17 @@ __device__ __forceinline__ void wait_previous(const Params& prm) {
   asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
+// Copies to shared memory behind the thread's back (16 bytes through L2 only,
+// 4 bytes); copy_async_wait: all of this thread's have landed
+__device__ __forceinline__ void copy_async16(uint32_t dst, const float* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void copy_async4(uint32_t dst, const float* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void copy_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void copy_async_wait() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
+
 // The mss prefix of sum m (0: A, 1: B, 2: C) of block blk, one lane per point:
 // MSS[o] = the levels' sums below o, from v[o * stride + m * 32 + lane] in
 // shared memory, added in the order of the levels.

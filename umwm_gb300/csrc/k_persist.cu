@@ -84,10 +84,11 @@ __device__ __forceinline__ void forcing_stage(const Params& prm, const Ptrs& P, 
 }
 
 // dynamic shared memory of the stages, one after another: the propagation's
-// level sums and rows in flight, the integration's cos(wdir - th) per warp
+// level sums and rows in flight, the integration's cos(wdir - th) and rows in
+// flight per warp
 template <int NP>
 static size_t persist_smem(int om) {
-  return sizeof(float) * std::max(adv_red_floats(om) + 4 * adv_ring_floats<NP>(), (size_t)4 * NP * 32);
+  return sizeof(float) * std::max(adv_red_floats(om) + 4 * adv_ring_floats<NP>(), 4 * (NP * 32 + integ_ring_floats<NP>()));
 }
 
 template <int NP, bool CURV>
@@ -131,7 +132,9 @@ __global__ void __launch_bounds__(128, UMWM_PERSIST_MINB)
     if (!bar_s(2)) return;
     if (blockIdx.x == 0) dts_body(prm, P, compute_rot, 0);
     if (!bar_s(3)) return;
-    for (int u = blockIdx.x * 4 + warp; u < nvb * NG; u += nb * 4) integ_body<NP>(prm, P, dirs, reinterpret_cast<float4*>(dsm) + warp * (NP / 4 * 32), u / NG, u % NG, 1);
+    for (int u = blockIdx.x * 4 + warp; u < nvb * NG; u += nb * 4) 
+      integ_body<NP, false>(prm, P, dirs, reinterpret_cast<float4*>(dsm) + warp * (NP / 4 * 32),
+                     dsm + 4 * NP * 32 + warp * integ_ring_floats<NP>(), u / NG, u % NG, 1);
     if (!bar_s(4)) return;
     for (int v = blockIdx.x; v < nvb; v += nb) {
       advect_body<NP, CURV, false, true, false>(prm, P, v, dirs, cw, dsm, dsm + adv_red_floats(prm.O));

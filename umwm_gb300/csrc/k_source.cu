@@ -33,7 +33,7 @@
 //   Bound by issue slots and latency at 15 warps per SM (128 registers).  The
 //   walk is downwards so that Snl's two levels are registers, not shared
 //   memory; a level's branch (below the cut-off, above, mixed) is taken once
-//   for the warp.  305 k points: 0.75 ms (before: 0.84); 171 points: 23 us in
+//   for the warp.  305 k points: 0.69 ms (before: 0.84); 171 points: 23 us in
 //   five chunks, 43 us in one (before: 47).
 #include <algorithm>
 
@@ -119,22 +119,29 @@ template <int NP, int WMAX, int MINB>
 __global__ void __launch_bounds__(WMAX * 32, MINB) k_integ(const Params prm, const Ptrs P, int nc) {
   // cos(wdir - th) per level chunk: the chunks' warps then need no barrier
   constexpr int NG = NP / integ_dirs<NP>(), NC = WMAX / NG;
+  extern __shared__ __align__(128) float dsm[];
   __shared__ float4 dirs[NP / 4 * DIR_ROWS], cw[NC * NP / 4 * 32];
   dir_fill<NP>(prm, reinterpret_cast<float*>(dirs));
   __syncthreads();
   const int w = threadIdx.x >> 5;
   wait_previous(prm);
-  integ_body<NP>(prm, P, adv_smem_u32(dirs), cw + (w / NG) * (NP / 4 * 32), blockIdx.x, w, nc);
+  integ_body<NP, MINB == 1>(prm, P, adv_smem_u32(dirs), cw + (w / NG) * (NP / 4 * 32), dsm + w * integ_ring_floats<NP>(),
+                 blockIdx.x, w, nc);
 }
 
 template <int NP, int WMAX, int MINB>
 static cudaError_t go_integ(const Params& prm, const Ptrs& P, int nc, cudaStream_t st) {
-  return launch_chained(k_integ<NP, WMAX, MINB>, prm.Ntot / 32, 32 * nc * (NP / integ_dirs<NP>()), 0, st, prm, P, nc);
+  constexpr size_t warp = integ_ring_floats<NP>() * sizeof(float);
+  const int warps = nc * (NP / integ_dirs<NP>());
+  static std::atomic<unsigned long long> done{0};
+  const cudaError_t e = allow_smem((const void*)k_integ<NP, WMAX, MINB>, WMAX * warp, done);
+  if (e != cudaSuccess) return e;
+  return launch_chained(k_integ<NP, WMAX, MINB>, prm.Ntot / 32, 32 * warps, warps * warp, st, prm, P, nc);
 }
 
 // prm.groups4: the levels of a block in several chunks (small models: the
 // walk over all levels is the time of the kernel there).  Else the register
-// budget of 15 warps per SM (128 registers, no spills), or of 18 where the
+// budget of 15 warps per SM (128 registers), or of 18 where the
 // blocks then fit one wave instead of two.  prm.minb_integ 3, 5: 12, 18 warps.
 template <int NP>
 static cudaError_t launch_integ_np(const Params& prm, const Ptrs& P, cudaStream_t st) {

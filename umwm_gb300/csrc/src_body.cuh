@@ -230,15 +230,29 @@ __device__ __forceinline__ void phys_body(const Params& prm, const Ptrs& P, int 
 // group g of D = NP/NG directions, levels [a, b).  The levels are walked
 // downwards: Snl at level o needs Sds e at o+1 and o+2, which are the two
 // levels before (kept in registers; a unit that does not start at the top
-// forms them first).  SAVE: this substep also stores its source terms for
-// stress('ocn').
+// forms them first).  A level's rows are copied to shared memory while the
+// level before is at work: read in place, half of a warp's time went by waiting
+// for them (756 -> 691 us at 305 k points, 384 -> 357 at 144 k; three stages
+// instead of two give no more).  EARLY: the e rows go to registers at the start
+// of a level (the forms of one CTA per SM: 45 us against 47 at 10 k points),
+// else a quad at a time, which spills less (713 against 691).  SAVE: this
+// substep also stores its source terms for stress('ocn').
 template <int NP>
 __host__ __device__ constexpr int integ_dirs() { return NP % 12 == 0 ? 12 : 8; }
 
-template <int NP, bool SAVE>
+// A level's rows, copied to shared memory during the level before: the warp's e
+// rows, the tables (IT_*) and the mss prefix, two stages per warp
+enum { IT_K, IT_CP0, IT_COTHKD, IT_LOGL2Z, IT_SDV, IT_FKOVG, IT_BF1R, IT_BF2R, IT_SBF, IT_CG0, IT_A, IT_B, IT_C, IT_ROWS };
+template <int NP>
+__host__ __device__ constexpr size_t integ_stage_floats() { return (size_t)(integ_dirs<NP>() + IT_ROWS) * 32; }
+template <int NP>
+__host__ __device__ constexpr size_t integ_ring_floats() { return 2 * integ_stage_floats<NP>(); }
+
+template <int NP, bool SAVE, bool EARLY>
 __device__ __forceinline__ void integ_unit(const Params& prm, const Ptrs& P, const Member& Mb, const Ctl* ctl, int blk,
-                                           uint32_t dirs, float4* cw, int g, int a, int b, bool chunked) {
+                                           uint32_t dirs, float4* cw, float* ring, int g, int a, int b, bool chunked) {
   constexpr int D = integ_dirs<NP>(), DQ = D / 4;
+  constexpr size_t SF = integ_stage_floats<NP>();
   const int lane = threadIdx.x & 31;
   const int O = prm.O, N = Mb.ghost;
   const int j = blk * 32 + lane;
@@ -260,10 +274,33 @@ __device__ __forceinline__ void integ_unit(const Params& prm, const Ptrs& P, con
   auto pf = [&](int o) {
     if (o >= a && lane == 0) {
       bulk_prefetch_l2(P.E + o * lstride + rb, D * 128);
-      if (g == 0) bulk_prefetch_l2(P.TAB + o * tstride + tb + T_SRC0 * 32, T_SRC_ROWS * 128);
+      if (g == 0) {
+        bulk_prefetch_l2(P.TAB + o * tstride + tb + T_SRC0 * 32, T_SRC_ROWS * 128);
+        if (!EARLY) bulk_prefetch_l2(P.MSS + ((size_t)blk * O + o) * 96, 384);
+      }
     }
   };
   for (int i = 1; i < PFD; ++i) pf(top - i);
+
+  const bool icy = __any_sync(0xffffffffu, s.sv != 0.f);
+  const uint32_t rg = adv_smem_u32(ring);
+  auto stage = [&](int o) {
+    const uint32_t d = rg + (uint32_t)((o & 1) * SF) * 4u;
+    const float* row = P.E + o * lstride + rb;
+#pragma unroll
+    for (int q = 0; q < DQ; ++q) copy_async16(d + q * 512 + lane * 16, row + q * 128);
+    const float* T = P.TAB + o * tstride + tb + lane;
+    const float* M3 = P.MSS + ((size_t)blk * prm.O + o) * 96 + lane;
+    const uint32_t t = d + D * 128 + lane * 4;
+    auto row4 = [&](int i, const float* src) { copy_async4(t + i * 128, src); };
+    row4(IT_K, T + T_K * 32), row4(IT_CP0, T + T_CP0 * 32), row4(IT_COTHKD, T + T_COTHKD * 32);
+    row4(IT_LOGL2Z, T + T_LOGL2Z * 32), row4(IT_SDV, T + T_SDV * 32), row4(IT_FKOVG, T + T_FKOVG * 32);
+    row4(IT_BF1R, T + T_BF1R * 32), row4(IT_BF2R, T + T_BF2R * 32), row4(IT_SBF, T + T_SBF * 32);
+    if (icy) row4(IT_CG0, T + T_CG0 * 32);
+    row4(IT_A, M3), row4(IT_B, M3 + 32), row4(IT_C, M3 + 64);
+    copy_async_commit();
+  };
+  stage(top);
 
   float2 d1[D / 2], d2[D / 2];  // Sds e at o+1, o+2
 #pragma unroll
@@ -274,23 +311,26 @@ __device__ __forceinline__ void integ_unit(const Params& prm, const Ptrs& P, con
     // before any writes
     if (chunked && o == b - 1) __syncthreads();
     pf(o - PFD);
-    const float* row = P.E + o * lstride + rb;
-    float4 e4[DQ];
+    copy_async_wait();  // this level's rows have landed
+    const float* const sp = ring + (o & 1) * SF;
+    auto erow = [&](int q) { return *reinterpret_cast<const float4*>(sp + q * 128 + lane * 4); };
+    float4 e4e[DQ];
+    if (EARLY) {
 #pragma unroll
-    for (int q = 0; q < DQ; ++q) e4[q] = *reinterpret_cast<const float4*>(row + q * 128);
-    const float* T = P.TAB + o * tstride + tb + lane;
-    const float* M3 = P.MSS + ((size_t)blk * prm.O + o) * 96 + lane;
-    const float kk = __ldg(T + T_K * 32), cp0 = __ldg(T + T_CP0 * 32);
-    const float coth = __ldg(T + T_COTHKD * 32);
-    const float U = fmaf(s.wi.ustar25, __ldg(T + T_LOGL2Z * 32), s.wi.wspd);
-    const float2 A = f2(M3[0]), B = f2(M3[32]), C = f2(M3[64]);
+      for (int q = 0; q < DQ; ++q) e4e[q] = erow(q);
+    }
+    const float* const T = sp + D * 32 + lane;
+    const float kk = T[IT_K * 32], cp0 = T[IT_CP0 * 32];
+    const float coth = T[IT_COTHKD * 32];
+    const float U = fmaf(s.wi.ustar25, T[IT_LOGL2Z * 32], s.wi.wspd);
+    const float2 A = f2(T[IT_A * 32]), B = f2(T[IT_B * 32]), C = f2(T[IT_C * 32]);
     // (the contractions are written out: the kernels that share this body are
     // to give the same bits)
-    const float k4 = pow4(kk), sdv = __ldg(T + T_SDV * 32);
+    const float k4 = pow4(kk), sdv = T[IT_SDV * 32];
     const float sA = prm.twopisds_fac * prm.f[o];
     const float2 U2 = f2(U), ncp = f2(-cp0);
-    const float2 gl = f2(__fmul_rn(s.wi.c1, __ldg(T + T_FKOVG * 32)));
-    const float sice = s.sv != 0.f ? __fmul_rn(2.f * __ldg(T + T_CG0 * 32), s.sv) : 0.f;
+    const float2 gl = f2(__fmul_rn(s.wi.c1, T[IT_FKOVG * 32]));
+    const float sice = s.sv != 0.f ? __fmul_rn(2.f * T[IT_CG0 * 32], s.sv) : 0.f;
     const float sdt = __fmul_rn(s.sdtc, kk);
     const bool prog = o < s.oc, write = o < b && valid;
     float* ES = P.ES + o * lstride + rb;
@@ -298,17 +338,18 @@ __device__ __forceinline__ void integ_unit(const Params& prm, const Ptrs& P, con
     // Sds is needed at the prognostic levels and at the two above them (Snl)
     const bool needs = SAVE || o < ocw + 2;
     const float2 lsk = f2(fmaf(prm.sds_power, lg2a(k4), lg2a(sA)));
-    const float2 b1 = f2(__ldg(T + T_BF1R * 32)), b2 = f2(__ldg(T + T_BF2R * 32));
-    const float2 nsk = f2(__fsub_rn(sice, __fadd_rn(__fadd_rn(__ldg(T + T_SBF * 32), sdt), sdv)));
+    const float2 b1 = f2(T[IT_BF1R * 32]), b2 = f2(T[IT_BF2R * 32]);
+    const float2 nsk = f2(__fsub_rn(sice, __fadd_rn(__fadd_rn(T[IT_SBF * 32], sdt), sdv)));
     // equilibrium above the cut-off, umwm_physics.F90:73-82: ef = (num / (sA t^2
     // coth))^(1/p) / k^4 as 2^((log2 num - 2 log2 t) / p + lt0)
     const float2 lt0 = f2(-fmaf(prm.inv_sds_power, lg2a(sA * coth), lg2a(k4)));
     const float2 ntail = f2(__fsub_rn(__fsub_rn(sice, sdt), sdv));
+    if (o > a) stage(o - 1);
     // One quad: PR some, TL some points of the warp prognostic, above their
     // cut-off; SD: Sds is formed
     auto quad = [&](auto PR, auto TL, auto SD, int q) {
       constexpr bool pr = decltype(PR)::value, tl = decltype(TL)::value, sdn = decltype(SD)::value;
-      const float4 cq = cwl[q * 32];
+      const float4 cq = cwl[q * 32], e4 = EARLY ? e4e[q] : erow(q);
       const F2x2 dc = dir4(dg, q, DIR_C), ds = dir4(dg, q, DIR_S);
       F2x2 dc2, ds2;
       if (tl || sdn) dc2 = dir4(dg, q, DIR_C2), ds2 = dir4(dg, q, DIR_S2);
@@ -316,7 +357,7 @@ __device__ __forceinline__ void integ_unit(const Params& prm, const Ptrs& P, con
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
         const int i = 2 * q + h;
-        const float2 e = h ? make_float2(e4[q].z, e4[q].w) : make_float2(e4[q].x, e4[q].y);
+        const float2 e = h ? make_float2(e4.z, e4.w) : make_float2(e4.x, e4.y);
         const float2 cw2 = h ? make_float2(cq.z, cq.w) : make_float2(cq.x, cq.y);
         float2 sds = f2(0.f), de = f2(0.f), snl = f2(0.f);
         if (sdn) {
@@ -388,9 +429,11 @@ __device__ __forceinline__ void integ_unit(const Params& prm, const Ptrs& P, con
 // Warp `w` of block blk's NG x nc warps: direction group fastest (a block's
 // tables are then shared through L1), then level chunk.  A CTA (or, with
 // nc = 1, any warp) runs it; with nc > 1 every warp of the CTA belongs to the
-// one block.  cw: NP/4 x 32 float4 of this chunk's warps.
-template <int NP>
-__device__ __forceinline__ void integ_body(const Params& prm, const Ptrs& P, uint32_t dirs, float4* cw, int blk, int w, int nc) {
+// one block.  cw: NP/4 x 32 float4 of this chunk's warps; ring: integ_ring_floats
+// of this warp.
+template <int NP, bool EARLY>
+__device__ __forceinline__ void integ_body(const Params& prm, const Ptrs& P, uint32_t dirs, float4* cw, float* ring, int blk, int w,
+                                           int nc) {
   constexpr int NG = NP / integ_dirs<NP>();
   const int g = w % NG, c = w / NG;
   const int tile = (blk * 32) / TILE;
@@ -404,9 +447,9 @@ __device__ __forceinline__ void integ_body(const Params& prm, const Ptrs& P, uin
   // keeps its source terms, and so does the model's first substep (its
   // spectrum output)
   if (P.src_sin && (ctl->done || ctl->first) && P.glob->save_src)
-    integ_unit<NP, true>(prm, P, Mb, ctl, blk, dirs, cw, g, a, b, nc > 1);
+    integ_unit<NP, true, EARLY>(prm, P, Mb, ctl, blk, dirs, cw, ring, g, a, b, nc > 1);
   else
-    integ_unit<NP, false>(prm, P, Mb, ctl, blk, dirs, cw, g, a, b, nc > 1);
+    integ_unit<NP, false, EARLY>(prm, P, Mb, ctl, blk, dirs, cw, ring, g, a, b, nc > 1);
 }
 
 }  // namespace umwm
