@@ -61,12 +61,9 @@ __device__ __forceinline__ bool grid_barrier(Global* g, unsigned expected, unsig
 }
 
 // The forcing interpolation of every member still inside the dtg, PREP_U
-// points per thread with their loads first (prep_points).  Measured on the
-// 1000x1000 random field (ms per substep, forcing / propagation / whole
-// substep): one point per thread 0.53 / 6.90 / 11.71; four points 0.20 /
-// 7.45 / 12.05 inlined and 0.20 / 7.51 / 12.40 as a separate function (the
-// larger register demand of the forcing stage costs the propagation more
-// than it saves).
+// points per thread with their loads first (prep_points).  One point per
+// thread: more overlap their latencies, but their registers cost the
+// propagation, which shares the budget, more than that saves.
 #ifndef UMWM_PERSIST_PREP_U
 #define UMWM_PERSIST_PREP_U 1
 #endif
@@ -93,7 +90,7 @@ static size_t persist_smem(int om) {
 
 template <int NP, bool CURV>
 #ifndef UMWM_PERSIST_MINB
-#define UMWM_PERSIST_MINB 4  // resident CTAs per SM (3, at 168 registers: 12.42 ms per substep against 11.71)
+#define UMWM_PERSIST_MINB 4  // resident CTAs per SM
 #endif
 __global__ void __launch_bounds__(128, UMWM_PERSIST_MINB)
     k_persist(const Params prm, const Ptrs P, unsigned expected, unsigned long long limit_ns) {
