@@ -53,14 +53,17 @@ constexpr int T_SRC0 = T_CP0, T_SRC_ROWS = T_BF2R + 1 - T_CP0;
 constexpr int TILE = 64;  // wet points of a tile (a member's points start on a tile boundary)
 
 // default levels ahead the spectral kernels prefetch the spectrum (and table)
-// rows into L2 (Params::pf_*, tunable); measured on 1000x1000: the
-// integration and the propagation are fastest at one level (two: +3 % and
-// +5 %, four: +13 % and +8 %), the dts pre-pass at two
+// rows into L2 (Params::pf_*, tunable).  The integration copies a level's rows
+// one level ahead, so the prefetch has to be two ahead to come before the copy:
+// 692 us with one, 650 with two, 644 with three at 305 k points, 181, 176 and
+// 176 at 86 k.  The propagation, 1.5 times as many rows in flight, loses with
+// more than one (305 k points 1153, 1162 and 1255 us; 86 k 280, 289 and 313);
+// the dts pre-pass is staged and prefetches only in its other form (two).
 #ifndef UMWM_PF_DIST_PHYS
 #define UMWM_PF_DIST_PHYS 2
 #endif
 #ifndef UMWM_PF_DIST_INTEG
-#define UMWM_PF_DIST_INTEG 1
+#define UMWM_PF_DIST_INTEG 2
 #endif
 #ifndef UMWM_PF_DIST_ADV
 #define UMWM_PF_DIST_ADV 1

@@ -33,7 +33,7 @@
 //   Bound by issue slots and latency at 15 warps per SM (128 registers).  The
 //   walk is downwards so that Snl's two levels are registers, not shared
 //   memory; a level's branch (below the cut-off, above, mixed) is taken once
-//   for the warp.  305 k points: 0.69 ms (before: 0.84); 171 points: 23 us in
+//   for the warp.  305 k points: 0.65 ms (before: 0.84); 171 points: 23 us in
 //   five chunks, 43 us in one (before: 47).
 #include <algorithm>
 

@@ -232,8 +232,9 @@ __device__ __forceinline__ void phys_body(const Params& prm, const Ptrs& P, int 
 // levels before (kept in registers; a unit that does not start at the top
 // forms them first).  A level's rows are copied to shared memory while the
 // level before is at work: read in place, half of a warp's time went by waiting
-// for them (756 -> 691 us at 305 k points, 384 -> 357 at 144 k; three stages
-// instead of two give no more).  EARLY: the e rows go to registers at the start
+// for them (756 -> 692 us at 305 k points, 384 -> 357 at 144 k, and 650 and 340
+// with the prefetch to L2 two levels ahead; three stages instead of two give no
+// more).  EARLY: the e rows go to registers at the start
 // of a level (the forms of one CTA per SM: 45 us against 47 at 10 k points),
 // else a quad at a time, which spills less (713 against 691).  SAVE: this
 // substep also stores its source terms for stress('ocn').
