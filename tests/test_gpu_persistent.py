@@ -112,3 +112,42 @@ def test_persistent_barrier_timeout(lib_built):
     U.umwm_run(case.start, case.stop)  # the context is usable and the run goes on
     _same(_state(U), ref)
     U.umwm_finalize()
+
+
+# stress('ocn') fields of a one-member model
+OCEAN = ("taux_ocntop", "tauy_ocntop", "taux_ocnbot", "tauy_ocnbot", "taux_snl", "tauy_snl", "epsx_ocn", "epsy_ocn",
+         "epsx_atm", "epsy_atm", "tailocnx", "tailocny", "taux1", "tauy1", "taux2", "tauy2", "taux3", "tauy3")
+
+
+@pytest.mark.parametrize("option,value", [("stress_ocn", 1), ("gust_seed", 7)])
+def test_option_between_persistent_runs(lib_built, option, value):
+    """An option that changes what the substeps are launched with takes effect
+    on a model whose persistent kernel has run before: the second run gives
+    the host loop's bits, ocean stresses included."""
+    from umwm_gb300 import configs
+
+    U = lib_built
+    case = configs.random_field(mm=40, nm=36, hours=1, dx=2000.0, dtg=600, gustiness=0.1)
+    for t in (600, 1200):
+        case.forcing[configs._time_str(case.start, t)] = case.forcing[case.start]
+    mid, end = (configs._time_str(case.start, t) for t in (600, 1200))
+
+    def run(persistent):
+        U.clear_inputs()
+        case.stage(U)
+        U.umwm_initialize(nml_text=case.nml)
+        U.set_option("use_graph", 0)
+        U.set_option("persistent", persistent)
+        U.umwm_run(case.start, mid)
+        U.set_option(option, value)
+        U.umwm_run(mid, end)
+        out = _state(U)[0][:4] + (tuple(U.get_field(n) for n in OCEAN) if option == "stress_ocn" else ())
+        gs = U.stat("persistent_graph")
+        U.umwm_finalize()
+        return out, gs
+
+    ref, _ = run(0)
+    got, gs = run(1)
+    assert gs in (1, -1)
+    for p, q in zip(got, ref):
+        np.testing.assert_array_equal(p, q)

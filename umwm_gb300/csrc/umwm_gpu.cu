@@ -1397,8 +1397,8 @@ bool dir_exists(const char* path) {
 }
 
 // Buffers of stress('ocn'): the last substep's source terms and the outputs.
-// Allocated on first use; a captured inner loop holds the old pointers and is
-// rebuilt.
+// Allocated on first use; the captured inner loops (the while node and the
+// persistent kernel's launch) hold the old pointers and are rebuilt.
 int ensure_ocn(Model& M) {
   if (M.P.src_sin) return UMWM_OK;
   const size_t spec = (size_t)M.prm.O * M.prm.P * M.prm.ldN;
@@ -1408,8 +1408,7 @@ int ensure_ocn(Model& M) {
   CU(D.alloc(&M.P.src_snl, spec, false));
   CU(D.alloc(&M.P.src_ust, (size_t)M.prm.ldN));
   CU(D.alloc(&M.P.ocn, (size_t)OCN_COUNT * M.prm.ldN));
-  if (M.graph_exec) { cudaGraphExecDestroy(M.graph_exec); M.graph_exec = nullptr; }
-  if (M.graph) { cudaGraphDestroy(M.graph); M.graph = nullptr; }
+  drop_graph(M);
   return UMWM_OK;
 }
 
@@ -2228,9 +2227,7 @@ int umwm_gpu_set_option(const char* name, double value) {
       return fail(UMWM_ERR_ARG, "gust_seed must be an integer in [0, 2^32)");
     M->gust_seed = (unsigned)value;
     M->prm.gust_seed = M->gust_seed;
-    // the captured inner loop holds the old parameters
-    if (M->graph_exec) { cudaGraphExecDestroy(M->graph_exec); M->graph_exec = nullptr; }
-    if (M->graph) { cudaGraphDestroy(M->graph); M->graph = nullptr; }
+    drop_graph(*M);  // the captured inner loops hold the old parameters
     return UMWM_OK;
   }
   if (s == "use_graph") { M->use_graph = value != 0; return UMWM_OK; }
