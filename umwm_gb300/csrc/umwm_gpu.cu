@@ -1400,13 +1400,13 @@ bool dir_exists(const char* path) {
 // Allocated on first use; the captured inner loops (the while node and the
 // persistent kernel's launch) hold the old pointers and are rebuilt.
 int ensure_ocn(Model& M) {
-  if (M.P.src_sin) return UMWM_OK;
+  if (M.P.ocn) return UMWM_OK;
   const size_t spec = (size_t)M.prm.O * M.prm.P * M.prm.ldN;
   Dev& D = *M.dev;
-  CU(D.alloc(&M.P.src_sin, spec, false));
-  CU(D.alloc(&M.P.src_sds, spec, false));
-  CU(D.alloc(&M.P.src_snl, spec, false));
-  CU(D.alloc(&M.P.src_ust, (size_t)M.prm.ldN));
+  // (those that a call short of memory left are kept, and the rest tried again)
+  for (float** p : {&M.P.src_sin, &M.P.src_sds, &M.P.src_snl})
+    if (!*p) CU(D.alloc(p, spec, false));
+  if (!M.P.src_ust) CU(D.alloc(&M.P.src_ust, (size_t)M.prm.ldN));
   CU(D.alloc(&M.P.ocn, (size_t)OCN_COUNT * M.prm.ldN));
   drop_graph(M);
   return UMWM_OK;
@@ -2037,7 +2037,7 @@ int umwm_gpu_get_field(const char* name, float* out, long n) {
   // source terms the last stress('ocn') step kept (its last substep's Sin,
   // Sds after cothkd and Snl), in the reference's (i, th, f) layout
   if (s == "ssin" || s == "sds" || s == "snl") {
-    if (!M->P.src_sin) return fail(UMWM_ERR_STATE, "get_field: " + s + " is kept by stress('ocn') steps only");
+    if (!M->P.ocn) return fail(UMWM_ERR_STATE, "get_field: " + s + " is kept by stress('ocn') steps only");
     const size_t cnt = (size_t)M->prm.O * M->prm.P * mh.N;
     if (need((long)cnt)) return UMWM_ERR_ARG;
     const float* src = s == "ssin" ? M->P.src_sin : s == "sds" ? M->P.src_sds : M->P.src_snl;
