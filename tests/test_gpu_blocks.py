@@ -113,3 +113,34 @@ def test_set_state_refreshes_the_mss_prefix(lib_built):
     assert np.abs(u1 - u0).max() <= 1e-5 * np.abs(u0).max()
     l2, p999, _ = spec_stats(F1, F0)
     assert l2 < 2e-6 and p999 < 1e-4, (l2, p999)
+
+
+@pytest.mark.parametrize("pm,om,kw", [(36, 37, {}), (36, 37, {"fice0": 0.5}), (8, 21, {}), (24, 30, {"fice0": 0.4}),
+                                      (48, 9, {})])
+def test_own_state_set_again_is_neutral(lib_built, pm, om, kw):
+    """A run that hands its own state back (another one in between) and goes on
+    gives the bits of the run that was never interrupted: the mss prefix and
+    the ice's level sums come from the spectrum alone, whoever formed them."""
+    from umwm_gb300 import configs
+
+    U = lib_built
+    case = configs.random_field(mm=40, nm=36, hours=1, dx=2000.0, pm=pm, om=om, **kw)
+
+    def run(swap):
+        U.clear_inputs()
+        case.stage(U)
+        U.umwm_initialize(nml_text=case.nml)
+        U.set_option("max_substeps", 4)
+        U.umwm_run(case.start, case.stop)
+        if swap:
+            F, u = U.get_state()
+            U.set_state(3.0 * F, u)
+            U.set_state(F, u)
+        U.set_option("max_substeps", 8)
+        U.umwm_run(case.start, case.stop)
+        out = U.get_state() + (U.get_screen(), U.get_field("physics_time_step"))
+        U.umwm_finalize()
+        return out
+
+    for a, b in zip(run(True), run(False)):
+        np.testing.assert_array_equal(a, b)

@@ -350,9 +350,7 @@ __device__ __forceinline__ void advect_body(const Params& prm, const Ptrs& P, in
         tx2 = __ffma2_rn(es2, c, tx2);
         ty2 = __ffma2_rn(es2, s, ty2);
         // the mss sums of the new spectrum (the source terms' prefix)
-        m0 = __fadd2_rn(m0, ef[h]);
-        m1 = __ffma2_rn(ef[h], dc2.a[h], m1);
-        m2 = __ffma2_rn(ef[h], ds2.a[h], m2);
+        mss_add(ef[h], dc2.a[h], ds2.a[h], m0, m1, m2);
       }
     }
     const float lf = icp * (wi.c1 * fkovg);

@@ -175,6 +175,14 @@ __device__ __forceinline__ void copy_async4(uint32_t dst, const float* src) {
 __device__ __forceinline__ void copy_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 __device__ __forceinline__ void copy_async_wait() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
 
+// Two directions' parts of a level's mss sums, e (1, cos 2th, sin 2th), even and
+// odd directions apart.  Whoever writes e adds them so.
+__device__ __forceinline__ void mss_add(float2 e, float2 c2, float2 s2, float2& m0, float2& m1, float2& m2) {
+  m0 = __fadd2_rn(m0, e);
+  m1 = __ffma2_rn(e, c2, m1);
+  m2 = __ffma2_rn(e, s2, m2);
+}
+
 // The mss prefix of sum m (0: A, 1: B, 2: C) of block blk, one lane per point:
 // MSS[o] = the levels' sums below o, from v[o * stride + m * 32 + lane] in
 // shared memory, added in the order of the levels.

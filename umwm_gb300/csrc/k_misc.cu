@@ -262,27 +262,29 @@ __global__ void __launch_bounds__(256) k_ref(const Params prm, float* __restrict
 }
 
 // The mss prefix (Ptrs::MSS) of blocks [b0, b0 + gridDim.x) from e: after a
-// state was set; the propagation keeps it from then on.
+// state was set; the propagation keeps it from then on.  A level's directions
+// are added as the propagation adds them (mss_add), so that a run goes on from
+// its own state, handed back, with the same bits.
 __global__ void __launch_bounds__(128) k_mss(const Params prm, const Ptrs P, int b0) {
   __shared__ float v[MAX_OM * 96];
   const int blk = b0 + blockIdx.x, lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
   const int j = blk * 32 + lane;
   for (int o = w; o < prm.O; o += nw) {
     const float4* r = reinterpret_cast<const float4*>(P.E + sidx(prm, o, 0, j));
-    float a = 0.f, b = 0.f, c = 0.f;
+    float2 m0 = f2(0.f), m1 = m0, m2 = m0;
     for (int q = 0; q < prm.P / 4; ++q) {
-      const float4 e = r[q * 32];
-      const float* c2 = prm.dc2th + 4 * q;
-      const float* s2 = prm.ds2th + 4 * q;
-      a += (e.x + e.y) + (e.z + e.w);
-      b += e.x * c2[0] + e.y * c2[1] + e.z * c2[2] + e.w * c2[3];
-      c += e.x * s2[0] + e.y * s2[1] + e.z * s2[2] + e.w * s2[3];
+      const float4 e4 = r[q * 32];
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+        mss_add(h ? make_float2(e4.z, e4.w) : make_float2(e4.x, e4.y),
+                make_float2(prm.dc2th[4 * q + 2 * h], prm.dc2th[4 * q + 2 * h + 1]),
+                make_float2(prm.ds2th[4 * q + 2 * h], prm.ds2th[4 * q + 2 * h + 1]), m0, m1, m2);
     }
     const float hk = P.TAB[tidx(prm, o, T_K3DK, j)] * (0.5f * prm.dth);
-    v[o * 96 + lane] = hk * a;
-    if (prm.ice_possible) P.ehs[((size_t)blk * prm.O + o) * 32 + lane] = P.TAB[tidx(prm, o, T_KDK, j)] * a;
-    v[o * 96 + 32 + lane] = hk * b;
-    v[o * 96 + 64 + lane] = hk * c;
+    v[o * 96 + lane] = hk * (m0.x + m0.y);
+    if (prm.ice_possible) P.ehs[((size_t)blk * prm.O + o) * 32 + lane] = P.TAB[tidx(prm, o, T_KDK, j)] * (m0.x + m0.y);
+    v[o * 96 + 32 + lane] = hk * (m1.x + m1.y);
+    v[o * 96 + 64 + lane] = hk * (m2.x + m2.y);
   }
   __syncthreads();
   if (w < 3) mss_prefix(prm, P, blk, w, v, 96);
