@@ -8,6 +8,7 @@
 // at 35 whatever the threads).
 #pragma once
 #include <cuda_runtime.h>
+#include <sys/mman.h>
 #include <unistd.h>
 
 #include <algorithm>
@@ -29,7 +30,9 @@ constexpr size_t COPY_PIECE = (size_t)32 << 20;
 class PageTouch {
  public:
   // Pages of [p, p + bytes), in pieces of `piece` bytes; nothing to do for
-  // memory that is pinned, managed or the device's, or for a small copy.
+  // memory that is pinned, managed or the device's, for a small copy, or where
+  // the pages are there (an array that the caller keeps: starting the threads
+  // took longer than it saved, 51 MB 0.64 ms against 0.43 without).
   PageTouch(void* p, size_t bytes, size_t piece) : p_(static_cast<char*>(p)), bytes_(bytes), piece_(piece) {
     if (bytes < MIN_BYTES || piece == 0) return;
     cudaPointerAttributes at{};
@@ -37,7 +40,7 @@ class PageTouch {
       cudaGetLastError();
       return;
     }
-    if (at.type != cudaMemoryTypeUnregistered) return;
+    if (at.type != cudaMemoryTypeUnregistered || !fresh()) return;
     const size_t cores = std::max(1u, std::thread::hardware_concurrency());
     const size_t nt = std::min({(size_t)8, std::max<size_t>(cores / 2, 1), bytes / MIN_BYTES});
     try {
@@ -62,6 +65,21 @@ class PageTouch {
 
  private:
   static constexpr size_t MIN_BYTES = (size_t)4 << 20;
+
+  // whether MIN_BYTES or more of the range has no page yet (or the kernel does not say)
+  bool fresh() const {
+    const size_t page = (size_t)sysconf(_SC_PAGESIZE);
+    const uintptr_t base = reinterpret_cast<uintptr_t>(p_);
+    unsigned char there[1024];
+    size_t missing = 0;
+    for (uintptr_t a = (base + page - 1) / page * page; a < base + bytes_; a += sizeof there * page) {
+      const size_t n = std::min(sizeof there, (base + bytes_ - a + page - 1) / page);
+      if (mincore(reinterpret_cast<void*>(a), n * page, there) != 0) return true;
+      for (size_t i = 0; i < n; ++i) missing += !(there[i] & 1);
+      if (missing * page >= MIN_BYTES) return true;
+    }
+    return false;
+  }
   // thread t's share of each piece: the pages that start in it.  A plain store,
   // of a byte that the copy is about to write: a load first (or an atomic or
   // with 0, which faults as a load) would map the zero page and then have every
