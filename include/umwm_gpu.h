@@ -301,7 +301,7 @@ int umwm_gpu_surrogate_train(int steps, int batch, double lr, unsigned long long
 int umwm_gpu_surrogate_eval(long first, long count, double* loss);
 
 /* Network output (n x 1344 f32) for input rows X (n x 1344 f32; rounded
- * to bf16 like every input). */
+ * to bf16 like every input).  Y may overlap X. */
 int umwm_gpu_surrogate_forward(const float* X, int n, float* Y);
 
 /* Mean-squared-error loss and its gradient (get_stat "surrogate_nparams"

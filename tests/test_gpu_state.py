@@ -91,3 +91,21 @@ def test_network_rows_in_pieces(lib_built):
     # the mean over both halves' rows
     assert abs(loss - 0.5 * (la + lb)) <= 0.02 * loss
     assert np.abs(g - 0.5 * (ga + gb)).max() <= 0.05 * np.abs(g).max()
+
+
+@pytest.mark.parametrize("shift", [0, 1, 6000])
+def test_network_rows_in_place(lib_built, shift):
+    """The outputs may overwrite the inputs: over the same rows, or `shift`
+    rows on (12000 rows are two pieces; the same batch gives the same bits)."""
+    U = lib_built
+    U.surrogate_init(37, 36, seed=3)
+    n, w = 12000, U.SURROGATE_WIDTH
+    X = np.random.default_rng(2).standard_normal((n, w), dtype=np.float32)
+    X[:, 1341:] = 0
+    ref = U.surrogate_forward(X)
+    for _ in range(3):
+        buf = np.empty((n + shift, w), np.float32)
+        buf[shift:] = X
+        rc = U.lib().umwm_gpu_surrogate_forward(buf[shift:].ctypes.data_as(FP), n, buf.ctypes.data_as(FP))
+        assert rc == 0
+        np.testing.assert_array_equal(buf[:n], ref)

@@ -579,6 +579,9 @@ int umwm_gpu_surrogate_forward(const float* X, int n, float* Y) {
                     S.Yf.as<float>(), nullptr, S.st)))
     return rc;
   const size_t total = (size_t)n * FPAD * sizeof(float);
+  // Y over X, in whole or in part: X has been read before Y's pages are written
+  const uintptr_t xa = reinterpret_cast<uintptr_t>(X), ya = reinterpret_cast<uintptr_t>(Y);
+  if (xa < ya + total && ya < xa + total) SCU(cudaStreamSynchronize(S.st));
   const PageTouch pages(Y, total, COPY_PIECE);  // while the device is at work
   for (size_t b = 0, c = 0; b < total; b += COPY_PIECE, ++c) {
     pages.wait(c);
