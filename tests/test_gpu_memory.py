@@ -40,3 +40,21 @@ def test_ocean_buffers_short_of_memory(lib_built):
 
     for a, b in zip(run(True), run(False)):
         np.testing.assert_array_equal(a, b)
+
+
+def test_network_batch_short_of_memory(lib_built):
+    import torch
+
+    U = lib_built
+    U.surrogate_init(37, 36, seed=3)
+    X = np.random.default_rng(4).standard_normal((30000, U.SURROGATE_WIDTH), dtype=np.float32)
+    X[:, 1341:] = 0
+    few = U.surrogate_forward(X[:256])
+    torch.cuda.empty_cache()
+    keep = torch.empty(torch.cuda.mem_get_info()[0] - (64 << 20), dtype=torch.uint8, device="cuda")
+    with pytest.raises(U.UmwmError):
+        U.surrogate_forward(X)
+    del keep
+    torch.cuda.empty_cache()
+    np.testing.assert_array_equal(U.surrogate_forward(X[:256]), few)
+    assert np.isfinite(U.surrogate_forward(X)).all()

@@ -107,6 +107,7 @@ double normal(uint64_t& x) {
 }
 
 int cuda_fail(cudaError_t e, const char* what) {
+  cudaGetLastError();  // reported: not to be met again by the check of a later launch
   return set_error(UMWM_ERR_CUDA, std::string("surrogate: ") + what + ": " + cudaGetErrorString(e));
 }
 

@@ -50,10 +50,15 @@ int fail(int code, const std::string& msg) {
   return code;
 }
 
+// (the error that is reported here is not to be met again by the check of a
+// later launch: one call short of memory would fail the next)
 #define CU(x)                                                                                   \
   do {                                                                                          \
     cudaError_t e_ = (x);                                                                       \
-    if (e_ != cudaSuccess) return fail(UMWM_ERR_CUDA, std::string(#x) + ": " + cudaGetErrorString(e_)); \
+    if (e_ != cudaSuccess) {                                                                    \
+      cudaGetLastError();                                                                       \
+      return fail(UMWM_ERR_CUDA, std::string(#x) + ": " + cudaGetErrorString(e_));              \
+    }                                                                                           \
   } while (0)
 
 unsigned enc_ord_h(float x) {
