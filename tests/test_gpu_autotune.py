@@ -99,3 +99,25 @@ def test_tma_forms_bit_identical(lib_built, option, value):
     assert c0 < 1000 and c1 // 1000 == value
     np.testing.assert_array_equal(F1, F0)
     np.testing.assert_array_equal(u1, u0)
+
+
+@pytest.mark.parametrize("mm,nm", [(64, 56), (170, 160)])  # with the split of the levels as the default, without
+def test_candidates_are_different_kernels(lib_built, mm, nm):
+    """No integration or propagation is measured under two names: a register
+    budget is a candidate only where it selects a kernel (not with the split of
+    the levels), and staged rows only where there is a form without."""
+    from umwm_gb300 import configs
+
+    U = lib_built
+    case = configs.random_field(mm=mm, nm=nm, hours=1, dx=2000.0)
+    U.clear_inputs()
+    case.stage(U)
+    U.umwm_initialize(nml_text=case.nml)
+    U.set_option("autotune", 2)
+    for k, budgets in (("integ", 2), ("advect", 3)):
+        cfg = [int(U.stat("tune_cfg:%s:%d" % (k, i))) for i in range(int(U.stat("tune_n:" + k)))]
+        assert len(set(cfg)) == len(cfg) and max(cfg) < 1000, (k, cfg)
+        assert len([c for c in cfg if c // 100 == 2]) == 2 * budgets, (k, cfg)
+        split = [c for c in cfg if c // 100 == 4]
+        assert len(split) == 2 and all((c // 10) % 10 == 0 for c in split), (k, cfg)
+    U.umwm_finalize()

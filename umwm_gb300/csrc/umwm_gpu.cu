@@ -317,7 +317,9 @@ void tune_set(Params& p, int k, const TuneCand& c) {
 }
 
 // Candidate lists.  Budgets have kernel instances only for 36 directions and
-// the 4-warp mapping (elsewhere a budget runs the default instance).
+// without the split of the levels (elsewhere a budget runs the default
+// instance, listed once by its prefetch distances).  The propagation stages its
+// rows in every form, so its staging option is not a candidate.
 void tune_start(Model& M, int mode) {
   Tuner& T = M.tune;
   T.mode = mode;
@@ -345,20 +347,16 @@ void tune_start(Model& M, int mode) {
         if (d36) minbs = g4 ? std::vector<int>{4, 5, 6} : std::vector<int>{5, 6, 7};
         pfs = {1, 2, 3};
       } else if (k == TK_INTEG) {
-        if (d36) minbs = g4 ? std::vector<int>{3, 4, 5} : std::vector<int>{3, 4};
+        // (with the split, fewer than 8 levels are not split)
+        if (d36 && !(g4 && p.O >= 8)) minbs = g4 ? std::vector<int>{3, 4, 5} : std::vector<int>{3, 4};
         pfs = {1, 2};
       } else {
-        if (d36 && !p.curvilinear) minbs = {3, 4, 5};
+        if (d36 && !p.curvilinear && !g4) minbs = {3, 4, 5};
         pfs = {1, 2};
       }
       for (int mb : minbs)
         for (int pf : pfs) K.cands.push_back({g4, mb, pf, 0});
-      // and with the rows staged (for the propagation the forms above again)
-      if (k == TK_ADVECT && d36 && !p.curvilinear && !g4)
-        for (int pf : pfs) {
-          K.cands.push_back({0, 3, pf, 1});
-          K.cands.push_back({0, 4, pf, 2});
-        }
+      // and with the rows staged
       if (k == TK_PHYS && d36 && !g4)
         for (int pf : {1, 2}) K.cands.push_back({0, 5, pf, 1});
     }
@@ -1428,8 +1426,13 @@ int enqueue_substep(Model& M, int compute_rot, int first, bool diag, const cudaG
   const Ptrs& P = M.P;
   const SubstepEnd end{first, dts_fused(prm) ? 1 : 0, loop ? 1 : 0, loop ? *loop : 0};
   CU(timed(M, K_PREP, [&] { return launch_prep(prm, P, compute_rot, M.max_nm, M.st); }));
-  CU(tuned(M, TK_PHYS, K_PHYS, [&] { return launch_source_phys(prm, P, compute_rot, end, M.st); }));
-  if (!end.fused) CU(timed(M, K_DTS, [&] { return launch_dts(prm, P, compute_rot, end, M.st); }));
+  // (the tuner times the pre-pass with what it leaves to a launch of its own)
+  const bool with_dts = M.tune.active && !end.fused;
+  CU(tuned(M, TK_PHYS, K_PHYS, [&] {
+    const cudaError_t e = launch_source_phys(prm, P, compute_rot, end, M.st);
+    return e == cudaSuccess && with_dts ? launch_dts(prm, P, compute_rot, end, M.st) : e;
+  }));
+  if (!end.fused && !with_dts) CU(timed(M, K_DTS, [&] { return launch_dts(prm, P, compute_rot, end, M.st); }));
   int rc;
   if (sur::active()) {
     // learned source step; points outside its energy budget fall back to
