@@ -24,12 +24,9 @@ __host__ __device__ constexpr size_t adv_ring_floats() { return (size_t)adv_stag
 
 template <bool COH>
 __device__ __forceinline__ void adv_copy16(uint32_t dst, const float* src) {
-  if (COH) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+  if (COH) copy_async16(dst, src);
   else asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
 }
-__device__ __forceinline__ void adv_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void adv_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 __device__ __forceinline__ float4 adv_lds(uint32_t a) {
   float4 v;
   asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
@@ -162,7 +159,7 @@ __device__ __forceinline__ void advect_body(const Params& prm, const Ptrs& P, in
         else if (o + nw < ocw) adv_copy16<COH>(d, P.ES + ro + (o + nw) * lstride);
       }
     }
-    adv_commit();
+    copy_async_commit();
   };
   auto lde = [](const float* a) { return COH ? __ldcg(a) : __ldg(a); };
 #pragma unroll
@@ -241,7 +238,7 @@ __device__ __forceinline__ void advect_body(const Params& prm, const Ptrs& P, in
     for (int q = 0; q < NQ; ++q) {
       const int p = 4 * q;
       if (AHEAD && q + 1 == NQ) tab(o + nw);
-      adv_wait<S - 2>();  // this quad's rows have landed
+      copy_async_wait<S - 2>();  // this quad's rows have landed
       const uint32_t d = rg + (uint32_t)(q % S) * 3072u;
       float4 ef4 = adv_lds(d + 512);  // e below the cut-off, ef above
       float2 ef[2] = {make_float2(ef4.x, ef4.y), make_float2(ef4.z, ef4.w)};
@@ -249,7 +246,7 @@ __device__ __forceinline__ void advect_body(const Params& prm, const Ptrs& P, in
       float4 nxt = make_float4(0.f, 0.f, 0.f, 0.f);
       if (anyp) {
         // th(p) = (p - (pm + 1) / 2) dth: sin th < 0 for p < pm/2, cos th < 0
-        // for p < pm/4 and p >= 3 pm/4 (checked at set-up: Params::swsign)
+        // for p < pm/4 and p >= 3 pm/4 (setup_params checks it)
         constexpr int H = NP / 2;
         const bool qE = CURV || p < H / 2 || p + 3 >= H + H / 2, qW = CURV || (p + 3 >= H / 2 && p < H + H / 2);
         const bool qN = CURV || p < H, qS = CURV || p + 3 >= H;

@@ -106,8 +106,6 @@ struct Params {
   int minb_phys, minb_integ, minb_adv;
   int pf_phys, pf_integ, pf_adv;
   int count_cut;     // the propagation counts the bins its non-negativity cut changes (Global::cut_count)
-  int swsign;        // the first pm/2 directions have sin th < 0, and of them the first pm/4 (and the last
-                     // pm/4 of all) cos th < 0: the propagation takes its upwind sides from the index
   int adv_tma;       // option "advect_tma" (no effect: the propagation stages its rows in every form)
   int phys_tma;      // the dts pre-pass stages its rows with bulk copies (option "phys_tma")
   float f[MAX_OM], dom[MAX_OM];

@@ -14,9 +14,6 @@ __device__ __forceinline__ float dec_ord_d(unsigned u) {
   return __uint_as_float((u & 0x80000000u) ? (u & 0x7fffffffu) : ~u);
 }
 
-// x^y for x >= 0 through the SFU (lg2/ex2); 0 for x == 0 (as pow does).
-__device__ __forceinline__ float pow_pos(float x, float y) { return exp2f(y * __log2f(x)); }
-
 // sheltering_coare35, umwm_sheltering.F90:49-79
 __device__ __forceinline__ float shelter_coare35(float w) {
   const float x1 = 15.f, x2 = 33.f, x3 = 60.f, y1 = 0.10f, y2 = 0.09f, y3 = 0.06f;
@@ -90,7 +87,7 @@ __device__ __forceinline__ float sin_fold(const Params& prm, float shelt, float 
 }
 
 // 2^x through the SFU (ex2.approx.ftz)
-__device__ __forceinline__ float ex2_approx(float x) {
+__device__ __forceinline__ float ex2a(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
@@ -165,7 +162,7 @@ __device__ __forceinline__ void wait_previous(const Params& prm) {
 }
 
 // Copies to shared memory behind the thread's back (16 bytes through L2 only,
-// 4 bytes); copy_async_wait: all of this thread's have landed
+// 4 bytes); copy_async_wait: all of this thread's but the last N groups have landed
 __device__ __forceinline__ void copy_async16(uint32_t dst, const float* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
 }
@@ -173,7 +170,8 @@ __device__ __forceinline__ void copy_async4(uint32_t dst, const float* src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
 }
 __device__ __forceinline__ void copy_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void copy_async_wait() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void copy_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
 // Two directions' parts of a level's mss sums, e (1, cos 2th, sin 2th), even and
 // odd directions apart.  Whoever writes e adds them so.

@@ -193,7 +193,7 @@ __global__ void __launch_bounds__(MW * 32) k_stokes(const Params prm, const Ptrs
         const float k2l = q4[64], is2 = q4[96], t = k2l * (dep + d);
         // |2 k (z + d)| > 50 or k d > 50: the deep-water profile
         const bool deep = is2 < 0.f || fabsf(t) > 50.f * log2e;
-        const float u = deep ? 2.f * ex2_approx(k2l * dep) : (0.5f * (ex2_approx(t) + ex2_approx(-t))) * is2;
+        const float u = deep ? 2.f * ex2a(k2l * dep) : (0.5f * (ex2a(t) + ex2a(-t))) * is2;
         su = fmaf(u, q4[0], su);
         sv = fmaf(u, q4[32], sv);
       }

@@ -7,11 +7,6 @@
 
 namespace umwm {
 
-__device__ __forceinline__ float ex2a(float x) {
-  float y;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
 __device__ __forceinline__ float lg2a(float x) {
   float y;
   asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -312,7 +307,7 @@ __device__ __forceinline__ void integ_unit(const Params& prm, const Ptrs& P, con
     // before any writes
     if (chunked && o == b - 1) __syncthreads();
     pf(o - PFD);
-    copy_async_wait();  // this level's rows have landed
+    copy_async_wait<0>();  // this level's rows have landed
     const float* const sp = ring + (o & 1) * SF;
     auto erow = [&](int q) { return *reinterpret_cast<const float4*>(sp + q * 128 + lane * 4); };
     float4 e4e[DQ];
