@@ -110,9 +110,10 @@ struct Params {
   int phys_tma;      // the dts pre-pass stages its rows with bulk copies (option "phys_tma")
   float f[MAX_OM], dom[MAX_OM];
   float th[MAX_PM], cth[MAX_PM], sth[MAX_PM], c2th[MAX_PM], s2th[MAX_PM];
-  // The spectral kernels' direction constants: those of a half turn's
-  // directions, negated for the others, so that opposite directions have the
-  // same rounding; and the mean sin and cos over the edge between p and p+1
+  // The spectral kernels' direction constants: those of a quarter turn's
+  // directions, turned exactly to the others, so that opposite and
+  // perpendicular directions have the same rounding; and the mean sin and cos
+  // over the edge between p and p+1
   float dcth[MAX_PM], dsth[MAX_PM], dc2th[MAX_PM], ds2th[MAX_PM], shs[MAX_PM], chs[MAX_PM];
   float depth[MAX_LM];
 };

@@ -649,19 +649,17 @@ int setup_params(Model& M) {
     p.c2th[q] = (float)std::cos(2.0 * (double)H.th[q]);
     p.s2th[q] = (float)std::sin(2.0 * (double)H.th[q]);
   }
-  // the spectral kernels' direction constants: the first half turn's, negated
-  // for the other.  The same for every domain, so that a member rounds alone as
-  // it does in a batch of any size.  (Built from a quarter turn, the cross-wind
-  // stress of a uniform basin, a small difference of large sums, is 1.5e-5 of
-  // its norm away from float64 at 37 k points instead of 1.0e-5, and 2.1e-5
-  // instead of 1.4e-5 at 171; elsewhere the two are alike.)
-  const int n = p.P / 2;
+  // the spectral kernels' direction constants: the first quarter turn's, turned
+  // exactly to the others.  The same for every domain, so that a member rounds
+  // alone as it does in a batch of any size
+  const int n = p.P / 4;
   for (int q = 0; q < p.P; ++q) {
-    const int g = q % n;
-    p.dcth[q] = q < n ? p.cth[g] : -p.cth[g];
-    p.dsth[q] = q < n ? p.sth[g] : -p.sth[g];
-    p.dc2th[q] = p.c2th[g];
-    p.ds2th[q] = p.s2th[g];
+    const int g = q / n;  // quarter turns from direction q % n
+    const float c = p.cth[q % n], s = p.sth[q % n], c2 = p.c2th[q % n], s2 = p.s2th[q % n];
+    p.dcth[q] = g == 0 ? c : g == 1 ? -s : g == 2 ? -c : s;
+    p.dsth[q] = g == 0 ? s : g == 1 ? c : g == 2 ? -s : -c;
+    p.dc2th[q] = g & 1 ? -c2 : c2;
+    p.ds2th[q] = g & 1 ? -s2 : s2;
   }
   for (int q = 0; q < p.P; ++q) {
     p.shs[q] = 0.5f * (p.dsth[q] + p.dsth[(q + 1) % p.P]);
