@@ -72,39 +72,3 @@ def test_ensemble_member_vs_oracle(lib_built, oracle_mod):
     l2, p999, mx = spec_stats(U.get_state()[0], o.get("e"))
     assert l2 < 1e-4 and p999 < 1e-3, (l2, p999, mx)
     U.umwm_finalize()
-
-
-def test_small_member_of_a_large_ensemble_matches_its_single_run(lib_built):
-    """A small domain gives the same bits alone (under one tile of 64 points per
-    SM) and as a member beside a large one (31 k points, over three)."""
-    from umwm_gb300 import configs
-
-    U = lib_built
-    small = configs.random_field(mm=40, nm=36, hours=1, dx=2000.0, seed=5)
-    large = configs.fetch_limited(mm=180, nm=178, hours=1, dx=2000.0, winds=True, currents=True)
-    zero = np.zeros((180, 178), np.float32)
-    for t in small.forcing:
-        large.forcing[t] = {"uw": zero + 10, "vw": zero + 3, "uc": zero + 0.2, "vc": zero}
-
-    def state():
-        F, u = U.get_state()
-        return F, u, U.get_field("taux"), U.get_field("physics_time_step"), U.get_screen()
-
-    U.clear_inputs()
-    small.stage(U)
-    U.umwm_initialize(nml_text=small.nml)
-    U.set_option("max_substeps", 6)
-    U.umwm_run(small.start, small.stop)
-    alone = state()
-    U.umwm_finalize()
-    U.clear_inputs()
-    for c in (small, large):
-        c.stage(U)
-        U.ensemble_add(c.nml)
-    U.ensemble_initialize()
-    U.set_option("max_substeps", 6)
-    U.umwm_run(small.start, small.stop)
-    U.select_member(0)
-    for a, b in zip(state(), alone):
-        np.testing.assert_array_equal(a, b)
-    U.umwm_finalize()

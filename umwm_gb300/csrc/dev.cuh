@@ -70,7 +70,8 @@ constexpr int TILE = 64;  // wet points of a tile (a member's points start on a 
 #endif
 
 // Direction counts with the small-model split of the levels over more warps
-// (options "direction_groups" and the like, value 4).
+// (options "direction_groups" and the like, value 4) and with direction
+// constants from a quarter turn.
 __host__ __device__ constexpr bool quarter_groups(int pm) {
   return pm % 4 == 0 && (pm / 4 == 4 || pm / 4 == 6 || pm / 4 == 8 || pm / 4 == 9 || pm / 4 == 12);
 }
@@ -110,10 +111,10 @@ struct Params {
   int phys_tma;      // the dts pre-pass stages its rows with bulk copies (option "phys_tma")
   float f[MAX_OM], dom[MAX_OM];
   float th[MAX_PM], cth[MAX_PM], sth[MAX_PM], c2th[MAX_PM], s2th[MAX_PM];
-  // The spectral kernels' direction constants: those of a quarter turn's
-  // directions, turned exactly to the others, so that opposite and
-  // perpendicular directions have the same rounding; and the mean sin and cos
-  // over the edge between p and p+1
+  // The spectral kernels' direction constants: those of the directions of a
+  // quarter (or half) turn, turned exactly to the others, so that opposite
+  // directions (and, with quarters, perpendicular ones) have the same rounding;
+  // and the mean sin and cos over the edge between p and p+1
   float dcth[MAX_PM], dsth[MAX_PM], dc2th[MAX_PM], ds2th[MAX_PM], shs[MAX_PM], chs[MAX_PM];
   float depth[MAX_LM];
 };

@@ -649,22 +649,6 @@ int setup_params(Model& M) {
     p.c2th[q] = (float)std::cos(2.0 * (double)H.th[q]);
     p.s2th[q] = (float)std::sin(2.0 * (double)H.th[q]);
   }
-  // the spectral kernels' direction constants: the first quarter turn's, turned
-  // exactly to the others.  The same for every domain, so that a member rounds
-  // alone as it does in a batch of any size
-  const int n = p.P / 4;
-  for (int q = 0; q < p.P; ++q) {
-    const int g = q / n;  // quarter turns from direction q % n
-    const float c = p.cth[q % n], s = p.sth[q % n], c2 = p.c2th[q % n], s2 = p.s2th[q % n];
-    p.dcth[q] = g == 0 ? c : g == 1 ? -s : g == 2 ? -c : s;
-    p.dsth[q] = g == 0 ? s : g == 1 ? c : g == 2 ? -s : -c;
-    p.dc2th[q] = g & 1 ? -c2 : c2;
-    p.ds2th[q] = g & 1 ? -s2 : s2;
-  }
-  for (int q = 0; q < p.P; ++q) {
-    p.shs[q] = 0.5f * (p.dsth[q] + p.dsth[(q + 1) % p.P]);
-    p.chs[q] = 0.5f * (p.dcth[q] + p.dcth[(q + 1) % p.P]);
-  }
   for (int l = 0; l < H.lm; ++l) p.depth[l] = H.depth[l];
   // launch configuration: default register budgets (0) and prefetch distances
   p.minb_phys = p.minb_integ = p.minb_adv = 0;
@@ -693,6 +677,21 @@ int init_device(Model& M) {
     CU(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
     p.nsm = nsm;
     if (quarter_groups(p.P) && p.ntiles <= nsm) p.groups4 = p.groups4_phys = p.adv_groups4 = 1;
+    // the direction constants: quarter turns on domains of under 192 points
+    // per SM, half turns on larger ones
+    const int turns = quarter_groups(p.P) && p.ntiles < 3 * nsm ? 4 : 2, n = p.P / turns;
+    for (int q = 0; q < p.P; ++q) {
+      const int g = (q / n) * (4 / turns);  // quarter turns from direction q % n
+      const float c = p.cth[q % n], s = p.sth[q % n], c2 = p.c2th[q % n], s2 = p.s2th[q % n];
+      p.dcth[q] = g == 0 ? c : g == 1 ? -s : g == 2 ? -c : s;
+      p.dsth[q] = g == 0 ? s : g == 1 ? c : g == 2 ? -s : -c;
+      p.dc2th[q] = g & 1 ? -c2 : c2;
+      p.ds2th[q] = g & 1 ? -s2 : s2;
+    }
+    for (int q = 0; q < p.P; ++q) {
+      p.shs[q] = 0.5f * (p.dsth[q] + p.dsth[(q + 1) % p.P]);
+      p.chs[q] = 0.5f * (p.dcth[q] + p.dcth[(q + 1) % p.P]);
+    }
   }
   M.dev.reset(new Dev());
   Dev& D = *M.dev;
