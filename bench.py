@@ -298,7 +298,6 @@ def run_ensemble(args):
 
     seq_ms = seq_bins = seq_sub = 0.0
     seq_ht = []
-    seq_groups = set()
     t_seq = time.perf_counter()
     for c in members:
         U.clear_inputs()
@@ -315,7 +314,6 @@ def run_ensemble(args):
         seq_bins += U.stat("bin_updates")
         seq_sub += U.dims()["substeps"] - s0
         seq_ht.append((k, U.get_field("ht")))
-        seq_groups.add((int(U.stat("config:integ")) // 100) % 10)
         U.umwm_finalize()
     t_seq = time.perf_counter() - t_seq
 
@@ -332,7 +330,6 @@ def run_ensemble(args):
         U.set_option("autotune", args.autotune)
     k = warm(args.autotune)
     tune = {kk: int(U.stat("config:" + kk)) for kk in ("phys", "integ", "advect")} if args.autotune else None
-    bat_groups = (int(U.stat("config:integ")) // 100) % 10
     launches0 = U.stat("launches")
     clocks = Clocks(local_rank)
     clocks.start()
@@ -354,12 +351,6 @@ def run_ensemble(args):
         if wm.any():
             hs_diff = max(hs_diff, float((np.abs(hb - htm)[wm] / htm[wm]).max()))
     U.umwm_finalize()
-    # members small enough to run alone with the quarter-turn direction
-    # mapping (chosen by size) round differently from the batch, which runs
-    # the half-turn mapping: then the arms agree to rounding, not bit for bit
-    if seq_groups != {bat_groups}:
-        same = None
-
     batched = bat_bins / (bat_ms / 1e3)
     sequential = seq_bins / (seq_ms / 1e3)
     line = {"metric": METRIC, "value": batched, "unit": UNIT, "n_gpus": 1, "steps": bat_outer,
@@ -377,7 +368,7 @@ def run_ensemble(args):
                            "member_substeps": seq_sub, "wall_s_incl_init": t_seq},
             "batched_over_sequential": batched / sequential,
             "bins_match": bool(bat_bins == seq_bins), "hs_bit_identical": same,
-            "hs_max_rel_diff": hs_diff, "direction_groups": {"sequential": sorted(seq_groups), "batched": bat_groups},
+            "hs_max_rel_diff": hs_diff,
             "gpu_launches": launches, "clocks": clk,
             "timing": "CUDA events on the model's stream around umwm_gpu_run of the timed dtg (both arms)"}
     if rank == 0:

@@ -209,7 +209,13 @@ int umwm_gpu_get_screen(double* out, long n, long* rows);
  * that suit large models; 4: to more of them; 4 needs pm % 4 == 0 and pm/4
  * in {4, 6, 8, 9, 12}; initialize picks 4 up to one 64-point tile per SM and
  * 2 above; results do not change), "advect_groups" (the same for the
- * propagation kernel alone), "gust_seed" (seed of the wind gust draws when
+ * propagation kernel alone), "direction_constants" (2 or 4: the direction
+ * cosines come from a half turn's directions or a quarter turn's, turned to
+ * the others; results differ by rounding; initialize takes 4 below three
+ * 64-point tiles per SM, where pm/4 is in {4, 6, 8, 9, 12}, and 2 elsewhere,
+ * so a small domain run alone gives the bits that it gives as a member of a
+ * large ensemble when it is set to the ensemble's choice, which
+ * umwm_gpu_get_stat reports under the same name), "gust_seed" (seed of the wind gust draws when
  * the namelist's gustiness > 0, umwm_forcing.F90:49-61; default 1: the
  * draws are a function of seed, substep, grid cell and component, so a run
  * repeats with its seed), "phys_groups" / "integ_groups" (the mapping of the
@@ -245,7 +251,7 @@ int umwm_gpu_set_option(const char* name, double value);
  * "device_free_bytes" (cudaMemGetInfo's free memory of the current device),
  * "cut_count" (bins the non-negativity cut changed since option
  * "count_cut" was set), "autotune_active", "autotune_done",
- * "autotune_substeps" (substeps measured),
+ * "autotune_substeps" (substeps measured), "direction_constants" (2 or 4),
  * "config:phys" / "config:integ" / "config:advect" (launch configuration in
  * use: direction groups * 100 + CTAs per SM * 10 + prefetch levels),
  * "tune_n:<kernel>", "tune_cfg:<kernel>:<i>", "tune_ms:<kernel>:<i>" (the

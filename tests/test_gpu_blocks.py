@@ -6,7 +6,7 @@ levels than warps, and the split of the levels, which must not change a bit.
 import numpy as np
 import pytest
 
-from helpers import run_gpu, run_oracle, spec_stats
+from helpers import lonlat_grid, run_gpu, run_oracle, spec_stats
 
 pytestmark = pytest.mark.gpu
 
@@ -144,3 +144,23 @@ def test_own_state_set_again_is_neutral(lib_built, pm, om, kw):
 
     for a, b in zip(run(True), run(False)):
         np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("pm,om,groups", [(8, 37, 2), (12, 20, 2), (16, 33, 2), (16, 33, 4), (24, 9, 4), (32, 25, 2), (32, 25, 4),
+                                          (48, 37, 2)])
+def test_curvilinear_direction_counts_vs_oracle(lib_built, oracle_mod, pm, om, groups):
+    """The propagation on a longitude-latitude grid (all four neighbours read,
+    the directions turned) with rings of two and of three slots; the tolerances
+    of the plain grid's test above."""
+    from umwm_gb300 import configs
+
+    U = lib_built
+    case = configs.random_field(mm=20, nm=17, hours=1, dx=2000.0, pm=pm, om=om, gridFromFile=True)
+    case.gridtopo["lon"], case.gridtopo["lat"] = lonlat_grid(20, 17)
+    run_gpu(U, case, max_substeps=2, groups=groups)
+    F, u = U.get_state()
+    U.umwm_finalize()
+    o = run_oracle(oracle_mod, case, 32, max_substeps=2)
+    l2, p999, _ = spec_stats(F, o.get("e"))
+    assert l2 < 2e-5 and p999 < 1e-3, (l2, p999)
+    assert np.abs(u - o.get("ustar")).max() <= 1e-3 * np.abs(o.get("ustar")).max()

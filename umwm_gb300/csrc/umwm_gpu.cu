@@ -159,6 +159,7 @@ struct Model {
   long long substeps = 0, max_substeps = -1;
   bool verbose = false, check_finite = false, use_graph = false;
   unsigned gust_seed = 1;  // seed of the wind gust draws (option "gust_seed")
+  int dir_turns = 0;       // the direction constants in use (dir_constants)
   // spectrum output (output_spectrum_nc): the points of namelists/spectrum.nml,
   // read at the first output, the time of that output (the files' names) and
   // the records written so far per point (each call rewrites the files)
@@ -566,6 +567,31 @@ int forcing_input(Model& M, MemberHost& mh, const std::string& key) {
   return UMWM_OK;
 }
 
+// The spectral kernels' direction constants: those of a quarter turn's
+// directions (turns 4) or a half turn's (2), turned exactly to the others.  The
+// two give results that differ by rounding (most in tauy of a uniform basin, a
+// small difference of large sums: 1.5e-5 and 1.0e-5 of its norm from float64 at
+// 37 k points, 2.1e-5 and 1.4e-5 at 171).  The size of the model chooses, so a
+// small member run alone and in a large batch gives the same bits only with the
+// same choice: option "direction_constants".
+void dir_constants(Model& M, int turns) {
+  Params& p = M.prm;
+  const int n = p.P / turns;
+  for (int q = 0; q < p.P; ++q) {
+    const int g = (q / n) * (4 / turns);  // quarter turns from direction q % n
+    const float c = p.cth[q % n], s = p.sth[q % n], c2 = p.c2th[q % n], s2 = p.s2th[q % n];
+    p.dcth[q] = g == 0 ? c : g == 1 ? -s : g == 2 ? -c : s;
+    p.dsth[q] = g == 0 ? s : g == 1 ? c : g == 2 ? -s : -c;
+    p.dc2th[q] = g & 1 ? -c2 : c2;
+    p.ds2th[q] = g & 1 ? -s2 : s2;
+  }
+  for (int q = 0; q < p.P; ++q) {
+    p.shs[q] = 0.5f * (p.dsth[q] + p.dsth[(q + 1) % p.P]);
+    p.chs[q] = 0.5f * (p.dcth[q] + p.dcth[(q + 1) % p.P]);
+  }
+  M.dir_turns = turns;
+}
+
 // Parameters shared by all members; members must agree on them.
 int setup_params(Model& M) {
   const HostModel& H = M.mem[0].H;
@@ -677,21 +703,8 @@ int init_device(Model& M) {
     CU(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
     p.nsm = nsm;
     if (quarter_groups(p.P) && p.ntiles <= nsm) p.groups4 = p.groups4_phys = p.adv_groups4 = 1;
-    // the direction constants: quarter turns on domains of under 192 points
-    // per SM, half turns on larger ones
-    const int turns = quarter_groups(p.P) && p.ntiles < 3 * nsm ? 4 : 2, n = p.P / turns;
-    for (int q = 0; q < p.P; ++q) {
-      const int g = (q / n) * (4 / turns);  // quarter turns from direction q % n
-      const float c = p.cth[q % n], s = p.sth[q % n], c2 = p.c2th[q % n], s2 = p.s2th[q % n];
-      p.dcth[q] = g == 0 ? c : g == 1 ? -s : g == 2 ? -c : s;
-      p.dsth[q] = g == 0 ? s : g == 1 ? c : g == 2 ? -s : -c;
-      p.dc2th[q] = g & 1 ? -c2 : c2;
-      p.ds2th[q] = g & 1 ? -s2 : s2;
-    }
-    for (int q = 0; q < p.P; ++q) {
-      p.shs[q] = 0.5f * (p.dsth[q] + p.dsth[(q + 1) % p.P]);
-      p.chs[q] = 0.5f * (p.dcth[q] + p.dcth[(q + 1) % p.P]);
-    }
+    // quarter turns on domains of under 192 points per SM, half turns on larger ones
+    dir_constants(M, quarter_groups(p.P) && p.ntiles < 3 * nsm ? 4 : 2);
   }
   M.dev.reset(new Dev());
   Dev& D = *M.dev;
@@ -2260,6 +2273,17 @@ int umwm_gpu_set_option(const char* name, double value) {
     drop_graph(*M);
     return UMWM_OK;
   }
+  if (s == "direction_constants") {
+    if (value != 2 && value != 4) return fail(UMWM_ERR_ARG, s + " must be 2 or 4");
+    if (value == 4 && !quarter_groups(M->prm.P))
+      return fail(UMWM_ERR_UNSUPPORTED, s + " 4 needs pm % 4 == 0 and pm/4 in {4, 6, 8, 9, 12}");
+    if (!M->on_device) return fail(UMWM_ERR_STATE, s + ": the model has no device state");
+    dir_constants(*M, (int)value);
+    drop_graph(*M);
+    CU(launch_mss(M->prm, M->P, 0, M->prm.ldN, M->st));  // the prefix is made with them
+    CU(cudaStreamSynchronize(M->st));
+    return UMWM_OK;
+  }
   // launch configuration of the spectral kernels (what the autotuner sets):
   // resident CTAs per SM of the register budget (0: the default instance; a
   // budget without an instance also runs the default) and prefetch distance
@@ -2344,6 +2368,7 @@ double umwm_gpu_get_stat(const char* name) {
     }
     return -1.0;
   }
+  if (s == "direction_constants") return (double)M->dir_turns;
   if (s == "autotune_active") return M->tune.active ? 1.0 : 0.0;
   if (s == "autotune_done") return M->tune.done ? 1.0 : 0.0;
   if (s == "autotune_substeps") return (double)M->tune.step;
