@@ -305,6 +305,7 @@ def run_ensemble(args):
         U.umwm_initialize(nml_text=c.nml)
         U.set_option("use_graph", 1)
         U.set_option("persistent", 1 if args.persistent else 0)
+        U.set_option("direction_constants", 2)  # the batch's: small domains alone would take the others
         if args.autotune:
             U.set_option("autotune", args.autotune)
         k = warm(args.autotune)
@@ -326,6 +327,7 @@ def run_ensemble(args):
     t_init = time.perf_counter() - t0
     U.set_option("use_graph", 1)
     U.set_option("persistent", 1 if args.persistent else 0)
+    U.set_option("direction_constants", 2)
     if args.autotune:
         U.set_option("autotune", args.autotune)
     k = warm(args.autotune)
@@ -743,7 +745,7 @@ def main():
     ap.add_argument("--member-hi", default="1000x600", help="largest ensemble member grid, MMxNM")
     ap.add_argument("--autotune", type=int, default=1, choices=[0, 1, 2],
                     help="library autotuner mode during the warm-up (1: register budgets and prefetch distances, "
-                         "results unchanged; 2: also the direction mappings)")
+                         "2: also the split of the levels over more warps; results unchanged)")
     ap.add_argument("--option", action="append", default=[], metavar="NAME=VALUE",
                     help="library option set after initialize (plain path), e.g. advect_groups=4")
     args = ap.parse_args()
@@ -804,10 +806,12 @@ def main():
         while U.stat("autotune_done") != 1 and U.dims()["substeps"] < t_sub + 200:
             advance_to(U.dims()["substeps"] + 1)
         cfg = {k: int(U.stat("config:" + k)) for k in ("phys", "integ", "advect")}
+        # resident CTAs of the instance that a budget number selects (the integration's CTAs have 3 warps,
+        # the propagation's 4, 8 and 6)
+        ctas = {"phys": {5: 5, 6: 6, 7: 7}, "integ": {3: 4, 4: 5, 5: 6}, "advect": {3: 3, 4: 2, 5: 2}}
         tune = {"mode": args.autotune, "substeps_measured": int(U.stat("autotune_substeps")),
-                "choice": {k: {"direction_groups": (v // 100) % 10, "ctas_per_sm": (v // 10) % 10 or "default",
-                               "prefetch_levels": v % 10,
-                               "own_rows_by_bulk_copy": {0: False, 1: "E* and e", 2: "E*"}.get(v // 1000, v // 1000)}
+                "choice": {k: {"direction_groups": (v // 100) % 10, "ctas_per_sm": ctas[k].get((v // 10) % 10, "default"),
+                               "prefetch_levels": v % 10, "rows_by_bulk_copy": v // 1000 == 1}
                            for k, v in cfg.items()},
                 "median_ms": {k: {str(int(U.stat("tune_cfg:%s:%d" % (k, i)))): round(U.stat("tune_ms:%s:%d" % (k, i)), 4)
                                   for i in range(int(U.stat("tune_n:" + k)))} for k in cfg}}
