@@ -201,8 +201,11 @@ int umwm_gpu_get_screen(double* out, long n, long* rows);
  * "use_graph" (run the inner loop as a CUDA graph with a device-side while
  * node: one host synchronisation per outer step instead of one per
  * substep; results are bit-identical), "kernel_timing" (CUDA-event time of
- * each kernel, read with umwm_gpu_get_stat "ms:<kernel>"; the inner loop
- * then runs host-driven), "device" (CUDA device of the next initialize),
+ * each kernel, read with umwm_gpu_get_stat "ms:<kernel>", launches with
+ * "count:<kernel>": prep, phys, dts, integ, advect, diag, stokes; the names
+ * sice and screen are kept and stay 0, their work being part of prep and
+ * advect, and so does dts on small models, where phys holds it; the sum over
+ * the names is the substep; the inner loop then runs host-driven), "device" (CUDA device of the next initialize),
  * "stress_ocn" (run stress('ocn') after every outer step: the last substep
  * of each step keeps its source terms, three more spectrum-sized arrays),
  * "direction_groups" (2: a block of 32 points' levels go to the few warps
@@ -215,30 +218,33 @@ int umwm_gpu_get_screen(double* out, long n, long* rows);
  * 64-point tiles per SM, where pm/4 is in {4, 6, 8, 9, 12}, and 2 elsewhere,
  * so a small domain run alone gives the bits that it gives as a member of a
  * large ensemble when it is set to the ensemble's choice, which
- * umwm_gpu_get_stat reports under the same name), "gust_seed" (seed of the wind gust draws when
- * the namelist's gustiness > 0, umwm_forcing.F90:49-61; default 1: the
+ * umwm_gpu_get_stat reports under the same name), "gust_seed" (seed of the
+ * wind gust draws when the namelist's gustiness > 0,
+ * umwm_forcing.F90:49-61; default 1: the
  * draws are a function of seed, substep, grid cell and component, so a run
  * repeats with its seed), "phys_groups" / "integ_groups" (the mapping of the
  * dts pre-pass or the integration alone), "minb_phys" / "minb_integ" /
- * "minb_advect" (the kernel instance: resident CTAs per SM its register
- * budget is sized for; 0 or a budget without a compiled instance: the
- * default) and "pf_phys" / "pf_integ" / "pf_advect" (frequency levels each
- * kernel prefetches into L2 ahead), "phys_tma" (default 1: the dts pre-pass
+ * "minb_advect" (the number of a compiled register budget, 36 directions and
+ * direction_groups 2: the pre-pass 5, 6, 7, its resident CTAs per SM where it
+ * does not stage its rows; the integration 3, 5 for 4, 6 CTAs of three warps;
+ * the propagation 3, 4, 5 for 3 CTAs of four warps, 2 of eight, 2 of six; 0
+ * or another number: the default) and "pf_phys" / "pf_integ" / "pf_advect"
+ * (frequency levels each kernel prefetches into L2 ahead), "phys_tma" (default 1: the dts pre-pass
  * stages its rows in shared memory with bulk copies; 36 directions; results
  * do not change), "advect_tma" (accepted; the propagation stages its rows in
  * every form),
  * "autotune" (0 off; 1: from the next substep
  * on, time the register budgets and prefetch distances of the three
  * spectral kernels on the model's own substeps, round-robin, and keep the
- * fastest of each; results do not change; 2: also the direction mappings,
- * which changes results by rounding only; choices are cached per domain
+ * fastest of each; 2: also the split of the levels (direction_groups);
+ * results do not change; choices are cached per domain
  * shape for the life of the process), "count_cut" (1: count the bins
  * whose negative ef the propagation cuts to 0 before e = ef, read with
  * umwm_gpu_get_stat "cut_count"; pm = 36 only), "persistent" (1: each
  * dtg's inner loop, every member, runs as one cooperative launch of the
  * persistent substep kernel with grid barriers between the stages; each
  * barrier wait is bounded (2 s) and one that runs out ends the run with
- * UMWM_ERR_TIMEOUT; pm = 36 and one direction mapping for all kernels;
+ * UMWM_ERR_TIMEOUT; pm = 36 and the same direction_groups for all kernels;
  * results are bit-identical to the other loops), "persistent_stall_test"
  * (1: the next persistent launch's barrier expects one CTA more than
  * launched, so its waits run out after 20 ms: for testing the time-out
@@ -253,7 +259,8 @@ int umwm_gpu_set_option(const char* name, double value);
  * "count_cut" was set), "autotune_active", "autotune_done",
  * "autotune_substeps" (substeps measured), "direction_constants" (2 or 4),
  * "config:phys" / "config:integ" / "config:advect" (launch configuration in
- * use: direction groups * 100 + CTAs per SM * 10 + prefetch levels),
+ * use: phys_tma / advect_tma * 1000 + direction groups * 100 + budget number
+ * (minb_*) * 10 + prefetch levels),
  * "tune_n:<kernel>", "tune_cfg:<kernel>:<i>", "tune_ms:<kernel>:<i>" (the
  * autotuner's candidates, their configurations and median times),
  * "persistent_graph" (1: the persistent launch is captured in a CUDA graph,

@@ -179,6 +179,8 @@ static cudaError_t launch_persist_t(const Params& prm, const Ptrs& P, int stall_
   return cudaLaunchCooperativeKernel((const void*)k_persist<NP, CURV>, dim3(grid), dim3(128), args, smem, st);
 }
 
+// (The kernel has a split of its own; that the others' agree is asked as it was
+// when they were mappings that rounded differently.)
 bool persist_supported(const Params& prm) {
   return prm.P == 36 && prm.groups4 == prm.groups4_phys && prm.groups4 == prm.adv_groups4;
 }

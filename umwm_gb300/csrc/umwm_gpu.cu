@@ -41,7 +41,7 @@ int g_device = -1;  // set_option("device", n) before initialize
 
 // Per-kernel CUDA-event timing on the launching stream (option "kernel_timing").
 // The sea-ice wave height and the screen line are parts of other kernels; their
-// statistics stay 0.
+// statistics stay 0, and so does that of dts where the pre-pass forms it.
 enum KName { K_PREP, K_SICE, K_PHYS, K_DTS, K_INTEG, K_ADVECT, K_DIAG, K_SCREEN, K_STOKES, K_NK };
 const char* const KNAMES[K_NK] = {"prep", "sice", "phys", "dts", "integ", "advect", "diag", "screen", "stokes"};
 
@@ -126,7 +126,7 @@ struct KernelTune {
 };
 enum { TK_PHYS = 0, TK_INTEG, TK_ADVECT, TK_N };
 struct Tuner {
-  int mode = 0;         // 0 off, 1 register budgets and prefetch, 2 also the direction mapping
+  int mode = 0;         // 0 off, 1 register budgets and prefetch, 2 also the split of the levels over more warps
   bool active = false;  // measuring
   bool done = false;    // a choice is in place (tuned or from the cache)
   int reps = 5;  // samples per candidate; the median decides (timing noise only adds time)
@@ -2253,7 +2253,7 @@ int umwm_gpu_set_option(const char* name, double value) {
   if (s == "use_graph") { M->use_graph = value != 0; return UMWM_OK; }
   if (s == "persistent") {
     if (value != 0 && !persist_supported(M->prm))
-      return fail(UMWM_ERR_UNSUPPORTED, "persistent needs pm = 36 and one direction mapping for all three kernels");
+      return fail(UMWM_ERR_UNSUPPORTED, "persistent needs pm = 36 and the same direction_groups for all three kernels");
     M->persistent = value != 0;
     return UMWM_OK;
   }
@@ -2372,8 +2372,9 @@ double umwm_gpu_get_stat(const char* name) {
   if (s == "autotune_active") return M->tune.active ? 1.0 : 0.0;
   if (s == "autotune_done") return M->tune.done ? 1.0 : 0.0;
   if (s == "autotune_substeps") return (double)M->tune.step;
-  // launch configuration in use, encoded as direction groups (2 or 4) * 100
-  // + CTAs per SM * 10 + prefetch levels (CTAs 0: the default instance)
+  // launch configuration in use, encoded as staging option * 1000 + split of
+  // the levels (2 or 4, as direction_groups) * 100 + budget number (minb_*) * 10
+  // + prefetch levels (budget 0: the default instance)
   if (s == "config:phys" || s == "config:integ" || s == "config:advect") {
     const int k = s == "config:phys" ? TK_PHYS : s == "config:integ" ? TK_INTEG : TK_ADVECT;
     const TuneCand c = tune_get(M->prm, k);
