@@ -188,3 +188,64 @@ def test_all_fallback_is_the_plain_path(lib_built):
     assert U.stat("surrogate_fallback") - f0 == U.stat("surrogate_points") - p0 > 0
     np.testing.assert_array_equal(Fs, Fp)
     np.testing.assert_array_equal(us, up)
+
+
+# direction quads in whole groups of three and with a remainder of one and two
+GRIDS = [(8, 37), (12, 25), (16, 33), (24, 30), (32, 25), (36, 37), (48, 27)]
+
+
+@pytest.mark.parametrize("pm,om", GRIDS)
+def test_features_other_grids(lib_built, mo, pm, om):
+    from umwm_gb300 import configs
+
+    U = lib_built
+    case = configs.random_field(mm=26, nm=23, hours=1, dx=2000.0, pm=pm, om=om)
+    U.clear_inputs()
+    case.stage(U)
+    U.umwm_initialize(nml_text=case.nml)
+    U.set_option("max_substeps", 2)
+    U.umwm_run(case.start, case.stop)
+    F = np.random.default_rng(pm + om).lognormal(-12.0, 4.0, (U.dims()["im"], pm, om)).astype(np.float32)
+    U.set_state(F)
+    Xg = U.surrogate_features()
+    ust = U.get_state()[1]
+    im = F.shape[0]
+    g = {k: U.get_field(k)[:im] for k in ("wdir", "wspd", "uc", "vc", "rhorat", "fice")}
+    Xo, _ = mo.features(F, g["wdir"].astype(np.float64), g["wspd"], ust, U.get_field("d")[:im], U.get_field("dts"),
+                        g["uc"], g["vc"], g["rhorat"], g["fice"], U.get_field("th").astype(np.float64),
+                        float(U.get_field("dth")))
+    U.umwm_finalize()
+    # as above: one bf16 step apart at most
+    bad = np.abs(Xg - Xo) > np.abs(Xo) * 2.0 ** -7 + 1e-6
+    assert bad.mean() < 1e-4, (bad.sum(), np.argwhere(bad)[:5])
+
+
+@pytest.mark.parametrize("pm,om", GRIDS[:-1])  # (48 directions exceed the apply step's shared memory: refused)
+def test_zero_network_keeps_the_spectrum(lib_built, mo, pm, om):
+    """A network whose output is zero changes no bin, at any level, of the
+    points that pass; a cold model's first substep has dts = 0, so neither does
+    the propagation: the spectrum comes back as it was set, up to the roundings
+    of (e + EPS) 2^0 - EPS, (e + ef) / 2 and 2 E* - e (2^-22 of e + EPS in all)."""
+    from umwm_gb300 import configs
+
+    U = lib_built
+    U.surrogate_init(om, pm, seed=3)
+    w = U.surrogate_get_params()
+    w[mo.OFF_W3:] = 0.0
+    U.surrogate_set_params(w)
+    case = configs.random_field(mm=26, nm=23, hours=1, dx=2000.0, pm=pm, om=om, restart=False)
+    U.clear_inputs()
+    case.stage(U)
+    U.umwm_initialize(nml_text=case.nml)
+    F = np.random.default_rng(pm * om).lognormal(-12.0, 4.0, (U.dims()["im"], pm, om)).astype(np.float32)
+    U.set_state(F)
+    U.set_option("surrogate", 1)
+    U.set_option("max_substeps", 1)
+    p0, f0 = U.stat("surrogate_points"), U.stat("surrogate_fallback")
+    U.umwm_run(case.start, case.stop)
+    pts, fb = U.stat("surrogate_points") - p0, U.stat("surrogate_fallback") - f0
+    G, dts = U.get_state()[0], U.get_field("dts")
+    U.set_option("surrogate", 0)
+    U.umwm_finalize()
+    assert pts == F.shape[0] and fb == 0 and dts == 0
+    assert (np.abs(G.astype(np.float64) - F) <= 2.0 ** -22 * (F + mo.EPS)).all()

@@ -13,7 +13,8 @@ namespace sur {
 
 namespace {
 
-constexpr int UNR = 12;                // spectrum loads in flight per warp in the bin loops
+constexpr int UNQ = 3;                 // quads of directions in flight per lane in the bin loops; k_apply at 69 k points:
+                                       // 319 us with 3, 354 with 1, 332 with 2, 328 with 5, 365 with 9
 constexpr int FLC = 8;                 // levels per chunk of k_features (one per warp)
 constexpr int FPITCHW = FLC * MAX_PM / 2 + 1;  // words per row of k_features' chunk tile (odd)
 
@@ -49,11 +50,11 @@ constexpr float GROWTH_SLACK = 0.02f;
 // Input rows of 32 points per CTA (8 warps).  Warp 0 finds each row's
 // point, rotation and extra features.  The spectrum part goes level chunk
 // by level chunk (FLC levels, FLC * pm columns of every row): warp w takes
-// level w of the chunk, lane = row, and walks the directions (UNR loads in
-// flight), writing the rotated bf16 features into a shared-memory tile; the
-// tile's row segments then go out as 32-bit words, coalesced along each
-// row.  For the inference rows (pts == nullptr, row r = point r) a level's
-// row of 32 points is one 128-byte line per direction.
+// level w of the chunk, lane = row, and walks the directions, four of a point
+// per load (UNQ loads in flight; single floats, 16 bytes apart in this layout,
+// took 209 us instead of 190 at 69 k points), writing the rotated bf16 features
+// into a shared-memory tile; the tile's row segments then go out as 32-bit
+// words, coalesced along each row.
 __global__ void __launch_bounds__(256) k_features(const Params prm, const Ptrs P, const int* pts, int n,
                                                   __nv_bfloat16* X, float* ecopy, int* shift) {
   __shared__ uint32_t tile[32 * FPITCHW];
@@ -100,18 +101,22 @@ __global__ void __launch_bounds__(256) k_features(const Params prm, const Ptrs P
     const int nl = min(FLC, prm.O - c0);  // levels of this chunk
     const int o = c0 + warp;
     if (warp < nl) {
-      const float* Er = ok ? P.E + sidx(prm, o, 0, j) : nullptr;  // direction p at Er[poff(p)]
-      int pr = s == 0 ? 0 : NP - s;                                  // rotated column of p = 0
-      for (int p0 = 0; p0 < NP; p0 += UNR) {
-        float ev[UNR];
+      const float4* Er = ok ? reinterpret_cast<const float4*>(P.E + sidx(prm, o, 0, j)) : nullptr;
+      int pr = s == 0 ? 0 : NP - s;  // rotated column of p = 0
+      for (int q0 = 0; q0 < NP / 4; q0 += UNQ) {
+        float4 ev[UNQ];
 #pragma unroll
-        for (int u = 0; u < UNR; ++u) ev[u] = (ok && p0 + u < NP) ? __ldg(Er + poff(p0 + u)) : 0.f;
+        for (int u = 0; u < UNQ; ++u) ev[u] = (ok && q0 + u < NP / 4) ? __ldg(Er + (q0 + u) * 32) : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-        for (int u = 0; u < UNR; ++u) {
-          if (p0 + u >= NP) break;
-          h[warp * NP + pr] = __float2bfloat16_rn(ok ? feature(ev[u]) : 0.f);
-          if (ecopy && r0 + lane < n) ecopy[(size_t)(r0 + lane) * F0 + o * NP + pr] = ev[u];
-          pr = pr + 1 == NP ? 0 : pr + 1;
+        for (int u = 0; u < UNQ; ++u) {
+          if (q0 + u >= NP / 4) break;
+          const float e4[4] = {ev[u].x, ev[u].y, ev[u].z, ev[u].w};
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            h[warp * NP + pr] = __float2bfloat16_rn(ok ? feature(e4[i]) : 0.f);
+            if (ecopy && r0 + lane < n) ecopy[(size_t)(r0 + lane) * F0 + o * NP + pr] = e4[i];
+            pr = pr + 1 == NP ? 0 : pr + 1;
+          }
         }
       }
     }
@@ -156,7 +161,9 @@ __global__ void k_targets(const Params prm, const Ptrs P, const int* pts, int n,
 // needs an atomic.  Pass 1 forms ef for every bin and writes E* = (e + ef)/2
 // and the monitor's sums; the points that pass get ef at the levels above
 // the cut-off in pass 2 (E* of the failing points is rewritten by the
-// fallback integration).
+// fallback integration).  Four directions of a point per load and store: single
+// floats took 398 us instead of 319 at 69 k points where no point passes, 547
+// instead of 433 where all do.
 __global__ void __launch_bounds__(256) k_apply(const Params prm, const Ptrs P, const __nv_bfloat16* Y, float tol,
                                                float tol_level, unsigned char* fb_pt, int* fb_tile,
                                                unsigned long long* counts) {
@@ -218,24 +225,32 @@ __global__ void __launch_bounds__(256) k_apply(const Params prm, const Ptrs P, c
     const float kdk = T[T_KDK * 32], logl2z = T[T_LOGL2Z * 32], cp0 = T[T_CP0 * 32], fkovg = T[T_FKOVG * 32];
     const bool tail = o >= wi.oc;
     float lv0 = 0.f, lv1 = 0.f;
-    for (int p0 = 0; p0 < NP; p0 += UNR) {
-      float ev[UNR];
+    const float4* Er = reinterpret_cast<const float4*>(P.E + sidx(prm, o, 0, j));
+    float4* Sr = reinterpret_cast<float4*>(P.ES + sidx(prm, o, 0, j));
+    for (int q0 = 0; q0 < NP / 4; q0 += UNQ) {
+      float4 ev[UNQ];
 #pragma unroll
-      for (int u = 0; u < UNR; ++u) ev[u] = (p0 + u < NP) ? P.E[sidx(prm, o, p0 + u, j)] : 0.f;
+      for (int u = 0; u < UNQ; ++u) ev[u] = q0 + u < NP / 4 ? Er[(q0 + u) * 32] : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-      for (int u = 0; u < UNR; ++u) {
-        const int p = p0 + u;
-        if (p >= NP) break;
-        const float e = ev[u];
-        float sp;
-        const float ef = step(p, e, logl2z, cp0, fkovg, tail, sp);
-        m0 += e * kdk;
-        m1 += ef * kdk;
-        w0 += fmaxf(e, 0.f) * sp * kdk;
-        w1 += ef * sp * kdk;
-        lv0 += fmaxf(e, 0.f);
-        lv1 += ef;
-        if (ok) P.ES[sidx(prm, o, p, j)] = 0.5f * (e + ef);
+      for (int u = 0; u < UNQ; ++u) {
+        const int q = q0 + u;
+        if (q >= NP / 4) break;
+        const float e4[4] = {ev[u].x, ev[u].y, ev[u].z, ev[u].w};
+        float es[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const float e = e4[i];
+          float sp;
+          const float ef = step(4 * q + i, e, logl2z, cp0, fkovg, tail, sp);
+          m0 += e * kdk;
+          m1 += ef * kdk;
+          w0 += fmaxf(e, 0.f) * sp * kdk;
+          w1 += ef * sp * kdk;
+          lv0 += fmaxf(e, 0.f);
+          lv1 += ef;
+          es[i] = 0.5f * (e + ef);
+        }
+        if (ok) Sr[q * 32] = make_float4(es[0], es[1], es[2], es[3]);
       }
     }
     lev0[o][lane] = lv0;
@@ -289,10 +304,16 @@ __global__ void __launch_bounds__(256) k_apply(const Params prm, const Ptrs P, c
     if (!(pass && o >= wi.oc)) continue;
     const float* T = P.TAB + tidx(prm, o, 0, j);
     const float logl2z = T[T_LOGL2Z * 32], cp0 = T[T_CP0 * 32], fkovg = T[T_FKOVG * 32];
-    for (int p = 0; p < NP; ++p) {
-      const size_t k = sidx(prm, o, p, j);
+    const size_t a = sidx(prm, o, 0, j);
+    for (int q = 0; q < NP / 4; ++q) {
+      const float4 e = reinterpret_cast<const float4*>(P.E + a)[q * 32];
       float sp;
-      P.EF[k] = step(p, P.E[k], logl2z, cp0, fkovg, true, sp);
+      float4 f;
+      f.x = step(4 * q, e.x, logl2z, cp0, fkovg, true, sp);
+      f.y = step(4 * q + 1, e.y, logl2z, cp0, fkovg, true, sp);
+      f.z = step(4 * q + 2, e.z, logl2z, cp0, fkovg, true, sp);
+      f.w = step(4 * q + 3, e.w, logl2z, cp0, fkovg, true, sp);
+      reinterpret_cast<float4*>(P.EF + a)[q * 32] = f;
     }
   }
 }
@@ -386,7 +407,7 @@ static int grid_for(size_t n, int block) {
 
 cudaError_t launch_features(const Params& prm, const Ptrs& P, const int* pts, int n, __nv_bfloat16* X,
                             float* ecopy, int* shift, cudaStream_t st) {
-  if (prm.O * prm.P + NEXTRA > FPAD || prm.P % 2) return cudaErrorInvalidValue;
+  if (prm.O * prm.P + NEXTRA > FPAD || prm.P % 4) return cudaErrorInvalidValue;
   if (n <= 0) return cudaSuccess;
   k_features<<<(n + 31) / 32, 256, 0, st>>>(prm, P, pts, n, X, ecopy, shift);
   return cudaGetLastError();
@@ -403,7 +424,7 @@ cudaError_t launch_apply(const Params& prm, const Ptrs& P, const __nv_bfloat16* 
                          unsigned char* fb_pt, int* fb_tile, unsigned long long* counts, cudaStream_t st) {
   // direction cosines [pm][32] and each warp's staged row segments [32][pm|1]
   const int smem = prm.P * 32 * 4 + 8 * 32 * (prm.P | 1) * 2;
-  if (smem > 48 * 1024 || prm.P % 2) return cudaErrorInvalidConfiguration;
+  if (smem > 48 * 1024 || prm.P % 4) return cudaErrorInvalidConfiguration;
   k_apply<<<prm.NB, 256, smem, st>>>(prm, P, Y, tol, tol_level, fb_pt, fb_tile, counts);
   return cudaGetLastError();
 }
